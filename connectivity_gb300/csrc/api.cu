@@ -96,6 +96,20 @@ gb_status ensure_ws(gb_ctx* c, int32_t n) {
   return GB_OK;
 }
 
+// Grows the context's contraction buffer to m edge pairs per half.
+gb_status ensure_con(gb_ctx* c, int64_t m) {
+  if (m <= c->con_cap) return GB_OK;
+  if (c->con_ws) {
+    cudaStreamSynchronize(c->stream);
+    cudaFree(c->con_ws);
+    c->con_ws = nullptr;
+    c->con_cap = 0;
+  }
+  CK(cudaMalloc(&c->con_ws, (size_t)m * 16), "contraction buffer");
+  c->con_cap = m;
+  return GB_OK;
+}
+
 void fill_params(const gb_opts* o, gb::RunParams& p) {
   gb_opts d;
   gb_opts_default(&d);
@@ -445,6 +459,15 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
   gb::RunParams p{};
   fill_params(o, p);
   p.count_unassigned = st != nullptr ? 1 : 0;
+  // Sparse graphs (up to five edges per vertex: lattices and road networks)
+  // may be contracted; the run kernel decides once it has seen the degrees.
+  // Denser graphs have hubs or short paths, where the searches are better.
+  if (kind == gb::kSCC && bv == nullptr && p.canonical && p.colour_mode == 2 && g->m > 0 &&
+      g->m <= 5 * (int64_t)g->n && p.fwbw_rounds == 1 && p.tune.expand_mode == 0) {
+    if ((s = ensure_con(c, g->m)) != GB_OK) return s;
+    w.con_edges = c->con_ws;
+    w.con_cap = c->con_cap;
+  }
   int grid = c->grid;
   if (o && o->grid_blocks > 0 && o->grid_blocks < grid) grid = o->grid_blocks;
   gb::GraphView gv{};
@@ -621,6 +644,7 @@ gb_status gb_ctx_destroy(gb_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   cudaFree(c->ws);
+  cudaFree(c->con_ws);
   cudaFree(c->d_ctl);
   cudaFree(c->d_sticky);
   cudaFree(c->d_tphase);

@@ -19,6 +19,8 @@ struct gb_ctx {
   int32_t cap_n = -1;           // workspace capacity in vertices
   void* ws = nullptr;
   gb::Work w{};
+  unsigned long long* con_ws = nullptr;  // contraction's edge pairs (2 x con_cap)
+  int64_t con_cap = 0;
   gb::Ctl* d_ctl = nullptr;
   gb::Ctl* h_ctl = nullptr;     // pinned
   int* d_sticky = nullptr;      // first error of any run since the last sync

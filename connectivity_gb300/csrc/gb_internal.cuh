@@ -56,6 +56,8 @@ enum Stat : int {
   kStNum = 16
 };
 
+constexpr int kConRounds = 64;  // cap on the contraction rounds of a run
+
 struct Ctl {
   // grid barrier word: arrivals so far (low 32 bits, never reset within a
   // run), bit 63 = an error was raised
@@ -93,7 +95,8 @@ struct Ctl {
   // steps: mode 8 = colours reset, 9 = propagation, 10 = roots,
   // 11 = same-colour marking, 12 = compaction; 15 = end of a kernel.
   // Trim: 16 = start, 17 = degree pass done, 18 = list counted, 19 = list
-  // written.
+  // written.  Contraction: 20 = start, 22 / 23 = a round of the
+  // grid / of one block, 24 = rounds done, 21 = end.
   struct Trace {
     unsigned long long t;
     unsigned long long t_mid;   // pull steps: end of the thread tier
@@ -111,6 +114,12 @@ struct Ctl {
   // Diagnostic: device time at which each block finished the thread tier of
   // the first pull step of the run.
   unsigned long long blk_t[256];
+  // contraction rounds (contract_device.cuh): per round the vertices and
+  // edges alive, the vertices merged and the edges logged so far
+  int32_t con_cnt[4][kConRounds + 2];
+  int32_t con_over;   // an array ran out
+  int32_t con_big;    // a vertex has too many edges
+  int32_t con_open;   // vertices left without a component
 };
 constexpr int kTrace = 128;
 constexpr int kBlkTimes = 256;
@@ -156,6 +165,8 @@ struct Work {
   int32_t* blk_i;         // per-block scratch (2 x grid size: counts, then pivot ids)
   unsigned long long* tphase;  // this run's 4 phase-boundary device times, or null
   long long* blk_l;       // per-block scratch (2 x grid size: pivot keys, then edge sums)
+  unsigned long long* con_edges;  // contraction: 2 x con_cap edge pairs, or null (not tried)
+  long long con_cap;
   Ctl* ctl;
 };
 
@@ -207,6 +218,11 @@ int max_coop_grid(int device);   // cooperative grid size for the run kernels
 cudaError_t launch_run_options(const GraphView& g, RunKind kind, const RunParams& p,
                                const Work& w, int grid, cudaStream_t stream);
 int run_options_blocks_per_sm();
+// The run with the contraction phase (kernels_contract.cu; SCC of a single
+// graph with Work::con_edges set), and the blocks per SM of its kernel.
+cudaError_t launch_run_contract(const GraphView& g, const RunParams& p, const Work& w, int grid,
+                                cudaStream_t stream);
+int run_contract_blocks_per_sm();
 
 // CSR construction (csr_build.cu).  build_csr sorts device edge arrays into
 // out- and (if in_off != null) in-CSR; *ids_ok = false if an id is outside

@@ -2,7 +2,7 @@
 // kernels, and the host launchers.  The device code of a run is in
 // run_device.cuh; the run kernels with the optional features compiled in
 // are in kernels_options.cu.
-#include "run_device.cuh"
+#include "run_kernel.cuh"
 
 namespace gb {
 namespace {
@@ -51,7 +51,8 @@ int max_coop_grid(int device) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
   int best = run_options_blocks_per_sm();
-  const int per[] = {run_blocks_per_sm(k_run<1, false>), run_blocks_per_sm(k_run<2, false>)};
+  const int per[] = {run_blocks_per_sm(k_run<1, false>), run_blocks_per_sm(k_run<2, false>),
+                     run_contract_blocks_per_sm()};
   for (int k : per) best = k < best ? k : best;
   if (best < 1) return 0;
   return best * sms;
@@ -79,6 +80,8 @@ cudaError_t launch_run(const GraphView& g, RunKind kind, const RunParams& p, con
   // graph walks the union of both
   if ((p.fwbw_rounds > 1 && g.batch.gid == nullptr) || p.tune.expand_mode != 0)
     e = launch_run_options(g, kind, p, w, grid, stream);
+  else if (kind == kSCC && w.con_edges != nullptr)
+    e = launch_run_contract(g, p, w, grid, stream);
   else
     e = (kind == kSCC || g.in.off == nullptr) ? coop(k_run<1, false>, grid, a, stream)
                                               : coop(k_run<2, false>, grid, a, stream);

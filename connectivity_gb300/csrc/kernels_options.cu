@@ -2,7 +2,7 @@
 // first, the edge-balanced push), in their own translation unit: the default
 // run kernels in kernels.cu keep their code whether or not this variant
 // exists.
-#include "run_device.cuh"
+#include "run_kernel.cuh"
 
 namespace gb {
 

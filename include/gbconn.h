@@ -120,7 +120,11 @@ typedef struct gb_opts {
                           edge between classes again; 2 (default) signature
                           rounds when at least 1048576 vertices are left after
                           FW-BW, else up to four colour rounds and signature
-                          rounds for what they leave.  Same labels. */
+                          rounds for what they leave.  Same labels.  With 2,
+                          a single graph of at most 5 n edges, none of whose
+                          valid vertices has more than 32 edges on a side, is
+                          first contracted (canonical = 1, fwbw_rounds = 1,
+                          expand_mode = 0): see colour_rounds of gb_stats. */
   int32_t wcc_mode;    /* WCC / CC of a device graph: 0 (default) the
                           reference's phases (trim, BFS from the pivot,
                           colour propagation, cc_main.cpp:184-245); 1 sampled
@@ -145,7 +149,9 @@ void gb_struct_sizes(int64_t sizes[3]);
 typedef struct gb_stats {
   double ms_trim, ms_reach, ms_colour, ms_canon, ms_total;
   int32_t pivot;          /* FW-BW source, -1 if none */
-  int32_t colour_rounds;
+  int32_t colour_rounds;  /* rounds of the colour phase, or of the contraction
+                             that found every component in its place (its time
+                             is part of ms_reach) */
   int64_t n_trim;         /* vertices labelled by trim */
   int64_t n_visit_fw;     /* vertices reached forward from the pivot */
   int64_t n_fwbw;         /* vertices labelled by FW-BW */
