@@ -192,7 +192,7 @@ gb_status graph_hints(gb_ctx* c, gb_graph* g) {
   if (!g->symmetric && !g->hint_in)
     CK(dev_alloc((void**)&g->hint_in, hb, true, c->stream), "hint allocation");
   CK(gb::build_hints(g->n, g->m, g->out_off, g->out_adj, g->in_off, g->in_adj, g->hint_out, g->hint_in,
-                     c->stream),
+                     &g->max_deg, c->stream),
      "hints");
   return GB_OK;
 }
@@ -374,16 +374,37 @@ gb_status run_small(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t* lab
   return GB_OK;
 }
 
-// WCC of a device graph by sampled union-find (cc_sampled_device): the
-// same bookkeeping as the one-block path (labels, events, status latch).
-gb_status run_sampled_cc(gb_ctx* c, const gb_graph* g, int32_t* labels, gb_stats* st,
-                         bool wait) {
+// WCC of a device graph of few edges per vertex and no hub takes the
+// union-find over its out-lists: it looks at every edge once, where the
+// searches settle a vertex of a power-law graph from one hint but pay a step
+// per hop on a wide graph (2048^2 lattice: 12.4 ms of searches, 0.25 ms).
+// Below four edges per vertex the searches run local rounds, and lose on
+// uniform random graphs too (1 M vertices, 3 M edges: 1.78 ms against 0.51;
+// with 4 M edges they take 0.36 and the union-find 0.75).  With hubs the
+// union-find loses (R-MAT of 1 M vertices and 4 edges each: 4.5 ms against
+// 0.28: the hubs' lists meet in a few blocks).  max_steps below the union-find's three
+// passes keeps the searches, which report the cap.
+constexpr int64_t kUnionMaxDeg = 64;
+bool use_union_cc(const gb_graph* g, const gb_opts* o) {
+  if (g->max_deg < 0 || g->max_deg > kUnionMaxDeg) return false;
+  if (o && (!o->canonical || o->fwbw_rounds > 1 || o->expand_mode == 1 ||
+            (o->max_steps > 0 && o->max_steps < 3)))
+    return false;
+  return g->m < (g->symmetric ? 8 : 4) * (int64_t)g->n;
+}
+
+// WCC of a device graph by union-find, sampled (cc_sampled_device) or of
+// every edge (cc_union_csr): the same bookkeeping as the one-block path
+// (labels, events, status latch).
+gb_status run_union_cc(gb_ctx* c, const gb_graph* g, int32_t* labels, gb_stats* st, bool wait,
+                       bool sampled) {
   const bool dev_labels = is_device_ptr(labels);
   if (!wait && !dev_labels) {
     gb_set_error("run: the asynchronous form needs device labels%s", "");
     return GB_ERR_INVALID;
   }
-  gb_status s = ensure_ws(c, g->n);
+  // (the workspace is needed for its label array only)
+  gb_status s = dev_labels ? GB_OK : ensure_ws(c, g->n);
   if (s != GB_OK) return s;
   int32_t* dl = dev_labels ? labels : c->w.label;
   cudaStream_t sm = c->stream;
@@ -392,13 +413,18 @@ gb_status run_sampled_cc(gb_ctx* c, const gb_graph* g, int32_t* labels, gb_stats
   CK(cudaMemsetAsync(c->d_tphase + 4 * (c->runs % gb_ctx::kRing), 0,
                      4 * sizeof(unsigned long long), sm),
      "memset");
+  if (!sampled) CK(cudaMemsetAsync(&c->d_ctl->uf_cross, 0, 8, sm), "memset");
   c->runs++;
   cudaEventRecord(ev[0], sm);
   // (a checked device graph: the id flag, err_where, stays clear)
-  CK(gb::cc_sampled_device(g->n, g->out_off, g->out_adj, g->symmetric ? nullptr : g->in_off,
-                           g->symmetric ? nullptr : g->in_adj, dl, &c->d_ctl->err_where,
-                           &c->d_ctl->err, sm),
-     "kernel launch");
+  if (sampled)
+    CK(gb::cc_sampled_device(g->n, g->out_off, g->out_adj, g->symmetric ? nullptr : g->in_off,
+                             g->symmetric ? nullptr : g->in_adj, dl, &c->d_ctl->err_where,
+                             &c->d_ctl->err, sm),
+       "kernel launch");
+  else
+    CK(gb::cc_union_csr(g->n, g->m, g->out_off, g->out_adj, dl, &c->d_ctl->uf_cross, sm),
+       "kernel launch");
   cudaEventRecord(ev[1], sm);
   cudaEventRecord(ev[4], sm);
   CK(gb::launch_latch(c->d_ctl, c->d_sticky, sm), "kernel launch");
@@ -443,7 +469,9 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
   if (g->n == 0) return GB_OK;
   if (bv == nullptr && use_small(g, o)) return run_small(c, g, kind, labels, o, st, wait);
   if (bv == nullptr && kind == gb::kWCC && o && o->wcc_mode == 1)
-    return run_sampled_cc(c, g, labels, st, wait);
+    return run_union_cc(c, g, labels, st, wait, true);
+  if (bv == nullptr && kind == gb::kWCC && use_union_cc(g, o))
+    return run_union_cc(c, g, labels, st, wait, false);
   gb_status s = ensure_ws(c, g->n);
   if (s != GB_OK) return s;
   const bool dev_labels = is_device_ptr(labels);
@@ -1165,8 +1193,9 @@ gb_status gb_cc(gb_ctx* c, const gb_graph* g, int32_t* labels, const gb_opts* o,
 
 namespace {
 // SCC / WCC of an edge list: small graphs take the one-block path straight
-// from the edges (no CSR build by radix sort, one launch); others get a
-// device graph that is built, run and freed.
+// from the edges (no CSR build by radix sort, one launch), WCC of larger ones
+// the union-find over the edges; SCC of larger ones gets a device graph that
+// is built, run and freed.
 gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int32_t* src,
                     const int32_t* dst, int32_t* labels, const gb_opts* o) {
   if (!c || n < 0 || m < 0 || (m > 0 && (!src || !dst)) || (n > 0 && !labels)) {
@@ -1179,7 +1208,12 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   gb_opts_default(&d);
   if (!o) o = gb::class_opts(c, n);
   if (!o) o = &d;
-  if (n > gb::kSmallMaxN || m >= (1ll << 31) || !o->small_path || !o->canonical) {
+  const bool small = n <= gb::kSmallMaxN && m < (1ll << 31) && o->small_path && o->canonical;
+  // WCC of a larger list: union-find over the edges, no CSR (its three
+  // passes against the step cap as in use_union_cc)
+  const bool uni = !small && kind == gb::kWCC && o->canonical &&
+                   !(o->max_steps > 0 && o->max_steps < 3);
+  if (!small && !uni) {
     gb_graph* g = nullptr;
     gb_status s = gb_graph_from_edges(c, n, m, src, dst, &g);
     if (s != GB_OK) return s;
@@ -1193,7 +1227,7 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   // one stream-ordered allocation: the edges (from host memory), the SCC
   // CSR built by the block (2m ints) and the labels (for host labels)
   const size_t edge_b = dev_edges ? 0 : (size_t)m * 8;
-  const size_t scr_b = kind == gb::kSCC ? (size_t)m * 8 : 0;
+  const size_t scr_b = kind == gb::kSCC ? (size_t)m * 8 : 0;  // (the one-block SCC)
   const size_t lab_b = dev_labels ? 0 : (size_t)n * 4;
   char* buf = nullptr;
   if (edge_b + scr_b + lab_b > 0)
@@ -1216,7 +1250,9 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   sd.labels = dev_labels ? labels : reinterpret_cast<int32_t*>(buf + edge_b + scr_b);
   const int32_t max_steps = o->max_steps > 0 ? o->max_steps : (1 << 30);
   if (e == cudaSuccess) e = cudaMemsetAsync(&c->d_ctl->err, 0, 2 * sizeof(int), sm);
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && uni)
+    e = gb::cc_union_edges(n, m, sd.src, sd.dst, sd.labels, &c->d_ctl->err, sm);
+  if (e == cudaSuccess && !uni)
     e = gb::launch_small(kind == gb::kSCC ? 0 : 1, sd, nullptr, 1, n, max_steps, &c->d_ctl->err,
                          sm, o->colour_mode);
   if (e == cudaSuccess && !dev_labels)

@@ -44,6 +44,7 @@ struct gb_graph {
   int32_t* in_adj = nullptr;
   int32_t* hint_out = nullptr;  // pull hints (null for the drop-in staging graph)
   int32_t* hint_in = nullptr;
+  int64_t max_deg = -1;         // largest total degree, found with the hints (-1: not known)
   bool pooled = false;          // arrays from the stream-ordered pool
   cudaStream_t pool_stream = nullptr;
 };

@@ -559,14 +559,23 @@ __device__ __forceinline__ uint8_t degree_key(long long d) {
   return (uint8_t)(32 + 8 * (e - 5) + (int)((dd >> (e - 3)) & 7));
 }
 
+// (and the largest total degree, into *most: one atomic per warp)
 __global__ void k_degree_key(int32_t n, const int64_t* out_off, const int64_t* in_off,
-                             uint8_t* key) {
+                             uint8_t* key, unsigned long long* most) {
+  long long best = 0;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
        v += (int64_t)gridDim.x * blockDim.x) {
     long long d = out_off[v + 1] - out_off[v];
     if (in_off) d += in_off[v + 1] - in_off[v];
     key[v] = degree_key(d);
+    best = d > best ? d : best;
   }
+  for (int o = 16; o; o >>= 1) {
+    const long long x = __shfl_xor_sync(0xffffffffu, best, o);
+    best = x > best ? x : best;
+  }
+  if ((threadIdx.x & 31) == 0 && (unsigned long long)best > *(volatile unsigned long long*)most)
+    atomicMax(most, (unsigned long long)best);
 }
 
 // The pull hint of a vertex: its neighbour of largest degree key, the first
@@ -614,7 +623,7 @@ struct HintSide {
 };
 
 // The lists the first pass fills.  count: [0] middle vertices, [1] heavy
-// vertices (ordinals), [2] heavy chunks.
+// vertices (ordinals), [2] heavy chunks, [3] the largest total degree.
 struct HintLists {
   int32_t* mid;
   int32_t* heavy;                // tag of each heavy ordinal
@@ -1096,7 +1105,8 @@ cudaError_t launch_latch(Ctl* ctl, int* sticky, cudaStream_t s) {
 
 cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int32_t* out_adj,
                         const int64_t* in_off, const int32_t* in_adj, int32_t* hint_out,
-                        int32_t* hint_in, cudaStream_t s) {
+                        int32_t* hint_in, int64_t* max_deg, cudaStream_t s) {
+  *max_deg = 0;
   if (n <= 0) return cudaSuccess;
   // the sides to build, the out-side first
   HintSide sd[2];
@@ -1131,7 +1141,7 @@ cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int3
     cudaFreeAsync(buf, s);
     return e;
   }
-  k_degree_key<<<grid_for(n), 256, 0, s>>>(n, out_off, in_off, deg);
+  k_degree_key<<<grid_for(n), 256, 0, s>>>(n, out_off, in_off, deg, L.count + 3);
   // the list passes: as many blocks as are resident at once on the SMs
   static const int gw_mid = resident_grid(k_hint_mid, kHintBlock);
   static const int gw_heavy = resident_grid(k_hint_heavy, kHintBlock);
@@ -1141,10 +1151,13 @@ cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int3
   k_hint_mid<<<gw_mid, kHintBlock, 0, s>>>(sd[0], sd[1], deg, L.mid, L.count);
   k_hint_heavy<<<gw_heavy, kHintBlock, 0, s>>>(sd[0], sd[1], deg, L);
   k_hint_slots<<<grid_for(L.heavy_cap), 256, 0, s>>>(sd[0], sd[1], L);
+  unsigned long long most = 0;
+  e = cudaMemcpyAsync(&most, L.count + 3, 8, cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(buf, s);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  *max_deg = e == cudaSuccess ? (int64_t)most : -1;
+  return e;
 }
 
 cudaError_t widen_offsets(const uint32_t* in, int64_t* out, int64_t count, cudaStream_t s) {

@@ -120,6 +120,7 @@ struct Ctl {
   int32_t con_over;   // an array ran out
   int32_t con_big;    // a vertex has too many edges
   int32_t con_open;   // vertices left without a component
+  unsigned long long uf_cross;  // union-find: edges that leave their range
 };
 constexpr int kTrace = 128;
 constexpr int kBlkTimes = 256;
@@ -313,6 +314,15 @@ cudaError_t cc_sampled(int32_t n, int64_t m, const uint32_t* h_off, const int32_
 cudaError_t cc_sampled_device(int32_t n, const int64_t* out_off, const int32_t* out_adj,
                               const int64_t* in_off, const int32_t* in_adj, int32_t* labels,
                               int* d_bad, int* d_err, cudaStream_t s);
+// Weakly connected components by union-find (unionfind.cu), smallest ids as
+// labels (device, n): of a device CSR (a directed graph's out-lists, or a
+// symmetric CSR), and of an edge list (*d_bad |= 1 on an id outside [0, n),
+// whose edge is left out).  Do not wait.
+// (d_cross: a zeroed word of scratch.)
+cudaError_t cc_union_csr(int32_t n, int64_t m, const int64_t* off, const int32_t* adj,
+                         int32_t* labels, unsigned long long* d_cross, cudaStream_t s);
+cudaError_t cc_union_edges(int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
+                           int32_t* labels, int* d_bad, cudaStream_t s);
 // *d_bad |= 1 when an id of adj[0, count) is outside [0, n).  Does not wait.
 cudaError_t check_ids_flag(int32_t n, const int32_t* adj, int64_t count, int* d_bad,
                            cudaStream_t s);
@@ -321,11 +331,11 @@ cudaError_t launch_localize(int32_t* labels, int32_t n, const int32_t* gid, cons
                             cudaStream_t s);
 // Pull hints: for every vertex, its neighbour of largest degree key (the
 // total degree, above 32 rounded down to eight steps per power of two) in
-// each CSR of m entries (hint_in may be null when in_off is).  Synchronises
-// the stream.
+// each CSR of m entries (hint_in may be null when in_off is).  *max_deg: the
+// largest total degree.  Synchronises the stream.
 cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int32_t* out_adj,
                         const int64_t* in_off, const int32_t* in_adj, int32_t* hint_out,
-                        int32_t* hint_in, cudaStream_t s);
+                        int32_t* hint_in, int64_t* max_deg, cudaStream_t s);
 // Seeded R-MAT edge list on the device for n vertices: edge_factor * n
 // candidate edges at scale ceil(log2 n), ids >= n, self-loops and duplicates
 // dropped, sorted by (src, dst); *d_src / *d_dst are cudaMallocAsync'd.

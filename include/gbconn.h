@@ -133,7 +133,12 @@ typedef struct gb_opts {
                           the sampled largest component link the rest; the
                           published Afforest scheme), which gb_run_cc uses on
                           a CSR in host memory.  Same labels.  Batches and
-                          graphs on the one-block path ignore it. */
+                          graphs on the one-block path ignore it.  With 0, a
+                          graph of fewer than 4 n edges (8 n entries of a
+                          symmetric CSR) and no vertex of total degree above
+                          64 takes a union-find over its edges (canonical = 1,
+                          fwbw_rounds = 1, expand_mode = 0, max_steps >= 3;
+                          the statistics then hold the times only). */
 } gb_opts;
 
 void gb_opts_default(gb_opts* o);
@@ -324,7 +329,8 @@ gb_status gb_cc(gb_ctx* ctx, const gb_graph* g, int32_t* labels, const gb_opts* 
  * entries (host or device).  A graph of at most 6144 vertices (small_path,
  * the default) runs in one thread block that builds its own CSR in shared
  * memory and scratch from the stream-ordered pool: one launch, no radix
- * sort.  Larger graphs are built as a device graph, run and freed.  Waits
+ * sort.  WCC of a larger list is a union-find over the edges; for SCC it is
+ * built as a device graph, run and freed.  Waits
  * for the result.  GB_ERR_INVALID: an id outside [0, n). */
 gb_status gb_scc_edges(gb_ctx* ctx, int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
                        int32_t* labels, const gb_opts* opts);
