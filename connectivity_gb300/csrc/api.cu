@@ -632,10 +632,11 @@ gb_status gb_ctx_create(int device, gb_ctx** out) {
     if ((r = cudaMallocHost(&c->h_tphase, pr)) != cudaSuccess) { s = cuda_fail(r, "phase ring"); break; }
     cudaMemset(c->d_tphase, 0, pr);
     std::memset(c->h_tphase, 0, pr);
-    if ((r = cudaMallocHost(&c->h_sticky, 2 * sizeof(int))) != cudaSuccess) { s = cuda_fail(r, "sticky"); break; }
+    if ((r = cudaMallocHost(&c->h_sticky, 4 * sizeof(int))) != cudaSuccess) { s = cuda_fail(r, "sticky"); break; }
     cudaMemset(c->d_sticky, 0, 2 * sizeof(int));
     std::memset(c->h_ctl, 0, sizeof(gb::Ctl));
-    c->h_sticky[0] = c->h_sticky[1] = 0;
+    c->h_sticky[0] = c->h_sticky[1] = c->h_sticky[2] = 0;
+    if ((r = cudaEventCreateWithFlags(&c->checked, cudaEventDisableTiming)) != cudaSuccess) { s = cuda_fail(r, "event"); break; }
     for (int k = 0; k < gb_ctx::kRing && s == GB_OK; ++k)
       for (int i = 0; i < 5 && s == GB_OK; ++i)
         if ((r = cudaEventCreate(&c->ev[k][i])) != cudaSuccess) s = cuda_fail(r, "event");
@@ -679,6 +680,7 @@ gb_status gb_ctx_destroy(gb_ctx* c) {
   if (c->h_tphase) cudaFreeHost(c->h_tphase);
   if (c->h_ctl) cudaFreeHost(c->h_ctl);
   if (c->h_sticky) cudaFreeHost(c->h_sticky);
+  if (c->checked) cudaEventDestroy(c->checked);
   for (auto& set : c->ev)
     for (auto& e : set)
       if (e) cudaEventDestroy(e);
@@ -760,7 +762,7 @@ int32_t gb_ctx_reach_trace2(gb_ctx* c, int64_t* t_ns, int32_t* count, int32_t* m
 }  // extern "C"
 
 gb_status gb::graph_from_edges(gb_ctx* c, int32_t n, int64_t m, const int32_t* src,
-                               const int32_t* dst, bool pooled, gb_graph** out) {
+                               const int32_t* dst, bool pooled, bool once, gb_graph** out) {
   if (!c || !out || n < 0 || m < 0 || (m > 0 && (!src || !dst))) return GB_ERR_INVALID;
   *out = nullptr;
   CK(cudaSetDevice(c->device), "cudaSetDevice");
@@ -783,7 +785,22 @@ gb_status gb::graph_from_edges(gb_ctx* c, int32_t n, int64_t m, const int32_t* s
     ds = ts;
     dd = tt;
   }
-  if (s == GB_OK) {
+  const bool part = once && gb::csr_part_fits(n, m);
+  if (s == GB_OK && part) {
+    void* scr = nullptr;
+    cudaError_t e = cudaMallocAsync(&scr, gb::csr_part_bytes(n, m), c->stream);
+    if (e == cudaSuccess) {
+      e = gb::csr_part_build(n, m, ds, dd, g->out_off, g->out_adj, g->in_off, g->in_adj, scr,
+                             c->h_sticky + 2, c->checked, c->stream);
+      cudaFreeAsync(scr, c->stream);
+    }
+    if (e == cudaSuccess) e = cudaEventSynchronize(c->checked);
+    if (e != cudaSuccess) s = cuda_fail(e, "CSR build");
+    else if (c->h_sticky[2]) {
+      gb_set_error("gb_graph_from_edges: %s", "vertex id outside [0, n)");
+      s = GB_ERR_INVALID;
+    }
+  } else if (s == GB_OK) {
     bool ok = true;
     cudaError_t e = gb::build_csr(n, m, ds, dd, g->out_off, g->out_adj, g->in_off, g->in_adj, c->stream, &ok);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -795,7 +812,7 @@ gb_status gb::graph_from_edges(gb_ctx* c, int32_t n, int64_t m, const int32_t* s
   }
   gb::dev_free(ts, pooled, c->stream);
   gb::dev_free(tt, pooled, c->stream);
-  if (s == GB_OK) s = graph_hints(c, g);
+  if (s == GB_OK && !once) s = graph_hints(c, g);
   if (s != GB_OK) {
     graph_free(g);
     delete g;
@@ -809,7 +826,7 @@ extern "C" {
 
 gb_status gb_graph_from_edges(gb_ctx* c, int32_t n, int64_t m, const int32_t* src,
                               const int32_t* dst, gb_graph** out) {
-  return gb::graph_from_edges(c, n, m, src, dst, false, out);
+  return gb::graph_from_edges(c, n, m, src, dst, false, false, out);
 }
 
 // Validates CSR arrays already on the device: off[0] == 0, off[n] == m,
@@ -1215,7 +1232,7 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
                    !(o->max_steps > 0 && o->max_steps < 3);
   if (!small && !uni) {
     gb_graph* g = nullptr;
-    gb_status s = gb_graph_from_edges(c, n, m, src, dst, &g);
+    gb_status s = gb::graph_from_edges(c, n, m, src, dst, true, true, &g);
     if (s != GB_OK) return s;
     s = gb::run_graph(c, g, kind, labels, o, nullptr, true, nullptr);
     gb_graph_destroy(g);

@@ -24,7 +24,8 @@ struct gb_ctx {
   gb::Ctl* d_ctl = nullptr;
   gb::Ctl* h_ctl = nullptr;     // pinned
   int* d_sticky = nullptr;      // first error of any run since the last sync
-  int* h_sticky = nullptr;      // pinned
+  int* h_sticky = nullptr;      // pinned; [2]: verdict of an edge list's id check
+  cudaEvent_t checked = nullptr;  // after that check
   static constexpr int kRing = 64;
   cudaEvent_t ev[kRing][5] = {};  // events of the last kRing runs: [0] start, [1] after the
                                   // run kernel, [4] end (after the statistics pass)
@@ -74,9 +75,12 @@ const gb_opts* class_opts(const gb_ctx* c, int64_t n);
 gb_status run_graph(gb_ctx* c, const gb_graph* g, RunKind kind, int32_t* labels,
                     const gb_opts* o, gb_stats* st, bool wait, const BatchView* bv);
 // Graph from an edge list; pooled graphs take their arrays from the
-// context stream's pool and free them on that stream.
+// context stream's pool and free them on that stream.  once: for a graph that
+// is run once and freed: its lists may come in any order and it gets no pull
+// hints (whose build costs more than they save one run); the build may still
+// be running when this returns.
 gb_status graph_from_edges(gb_ctx* c, int32_t n, int64_t m, const int32_t* src,
-                           const int32_t* dst, bool pooled, gb_graph** out);
+                           const int32_t* dst, bool pooled, bool once, gb_graph** out);
 // Batch from a concatenated global-id edge list (host or device).
 gb_status batch_create(gb_ctx* c, int32_t count, const int64_t* vbase, int64_t m,
                        const int32_t* src, const int32_t* dst, bool check_edges, bool pooled,

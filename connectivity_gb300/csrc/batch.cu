@@ -94,9 +94,9 @@ gb_status batch_finish(gb_ctx* c, gb_batch* b, const int32_t* d_src, const int32
       return GB_ERR_INVALID;
     }
   }
-  unsigned long long mo = 0, mi = 0;
-  CKB(gb::max_degree(n, b->g->out_off, c->stream, &mo), "batch degrees");
-  CKB(gb::max_degree(n, b->g->in_off, c->stream, &mi), "batch degrees");
+  unsigned long long md[2] = {0, 0};
+  CKB(gb::max_degrees(n, b->g->out_off, b->g->in_off, c->stream, md), "batch degrees");
+  const unsigned long long mo = md[0], mi = md[1];
   int ib = bits_of((unsigned long long)(n > 1 ? n - 1 : 1));
   b->id_bits = ib > 0 ? ib : 1;
   b->score_bits_scc = bits_of(mo * mi);
@@ -125,7 +125,7 @@ gb_status batch_from_union(gb_ctx* c, int32_t count, const int64_t* vbase, int64
   b->pooled = pooled;
   b->pool_stream = c->stream;
   b->vbase.assign(vbase, vbase + count + 1);
-  gb_status s = gb::graph_from_edges(c, (int32_t)vbase[count], m, src, dst, pooled, &b->g);
+  gb_status s = gb::graph_from_edges(c, (int32_t)vbase[count], m, src, dst, pooled, pooled, &b->g);
   if (s == GB_OK) {
     // the checks need device copies of the edges; from_edges already
     // validated ids against n, so only the within-graph rule remains

@@ -120,6 +120,7 @@ struct Ctl {
   int32_t con_over;   // an array ran out
   int32_t con_big;    // a vertex has too many edges
   int32_t con_open;   // vertices left without a component
+  int32_t con_may;    // sampled vertices that the first round may merge
   unsigned long long uf_cross;  // union-find: edges that leave their range
 };
 constexpr int kTrace = 128;
@@ -231,6 +232,15 @@ int run_contract_blocks_per_sm();
 cudaError_t build_csr(int32_t n, int64_t m, const int32_t* d_src, const int32_t* d_dst,
                       int64_t* out_off, int32_t* out_adj, int64_t* in_off, int32_t* in_adj,
                       cudaStream_t s, bool* ids_ok);
+// Out- and in-CSR with the lists in no particular order (csr_part.cu), for
+// graphs that csr_part_fits; scratch of csr_part_bytes.  *h_bad (pinned) is 1
+// for an id outside [0, n) once `checked` has passed; the CSR is not written
+// then.  Does not wait.
+bool csr_part_fits(int32_t n, int64_t m);
+size_t csr_part_bytes(int32_t n, int64_t m);
+cudaError_t csr_part_build(int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
+                           int64_t* out_off, int32_t* out_adj, int64_t* in_off, int32_t* in_adj,
+                           void* scratch, int* h_bad, cudaEvent_t checked, cudaStream_t s);
 // Sets *bad when off[0] != 0, off[n] != m, offsets decrease or an id is
 // outside [0, n).  Synchronises the stream.
 cudaError_t check_csr(int32_t n, int64_t m, const int64_t* off, const int32_t* adj,
@@ -352,7 +362,9 @@ cudaError_t batch_gid(int32_t n, const int64_t* d_vbase, int32_t count, int32_t*
 // Sets *bad if an edge joins two graphs.  Synchronises the stream.
 cudaError_t batch_check_within(const int32_t* src, const int32_t* dst, int64_t m,
                                const int32_t* gid, cudaStream_t s, int* bad);
-// Largest degree of a CSR.  Synchronises the stream.
-cudaError_t max_degree(int32_t n, const int64_t* off, cudaStream_t s, unsigned long long* out);
+// Largest degree of each of two CSRs, into out[0..1].  Synchronises the
+// stream.
+cudaError_t max_degrees(int32_t n, const int64_t* off0, const int64_t* off1, cudaStream_t s,
+                        unsigned long long* out);
 
 }  // namespace gb

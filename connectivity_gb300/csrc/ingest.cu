@@ -246,7 +246,7 @@ gb_status from_text(gb_ctx* c, FILE* f, const char* path, int64_t size, int chun
   }
   cudaFreeAsync(text, s);
   text = nullptr;
-  st = gb::graph_from_edges(c, n, m, src, dst, false, out);
+  st = gb::graph_from_edges(c, n, m, src, dst, false, false, out);
   cleanup();
   return st;
 }
@@ -270,7 +270,7 @@ gb_status from_binary(gb_ctx* c, FILE* f, const char* path, int64_t size, gb_gra
   }
   gb_status st = stream_to_device(c, f, (unsigned char*)src, m * 4, path);
   if (st == GB_OK) st = stream_to_device(c, f, (unsigned char*)dst, m * 4, path);
-  if (st == GB_OK) st = gb::graph_from_edges(c, n, m, src, dst, false, out);
+  if (st == GB_OK) st = gb::graph_from_edges(c, n, m, src, dst, false, false, out);
   cudaFreeAsync(src, s);
   cudaFreeAsync(dst, s);
   cudaStreamSynchronize(s);
