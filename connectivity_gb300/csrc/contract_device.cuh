@@ -84,8 +84,15 @@ struct ConGrid {
   __device__ __forceinline__ long long threads() const {
     return (long long)gridDim.x * blockDim.x;
   }
+  // Loads go through L1, where the words every warp ends at (a large
+  // component's root, a hub's extremes) are served per SM instead of one
+  // request at a time by L2.  The barrier after each pass drops what L1 holds
+  // from before it; within a pass a stale value is an older extreme or
+  // ancestor, which costs work only.  fresh() is for the union-find.
   template <class T>
-  static __device__ __forceinline__ T ld(const T* p) { return __ldcg(p); }
+  static __device__ __forceinline__ T ld(const T* p) { return __ldca(p); }
+  template <class T>
+  static __device__ __forceinline__ T fresh(const T* p) { return __ldcg(p); }
   __device__ __forceinline__ bool sync(int where) const {
     if (st->s - st->s0 >= max_steps) {
       set_err(c, kErrIterLimit, where);
@@ -102,6 +109,8 @@ struct ConBlock {
   __device__ __forceinline__ long long threads() const { return blockDim.x; }
   template <class T>
   static __device__ __forceinline__ T ld(const T* p) { return *(const volatile T*)p; }
+  template <class T>
+  static __device__ __forceinline__ T fresh(const T* p) { return *(const volatile T*)p; }
   static __device__ __forceinline__ int2 ld(const int2* p) {
     const volatile int* q = reinterpret_cast<const volatile int*>(p);
     return make_int2(q[0], q[1]);
@@ -178,11 +187,15 @@ __device__ __forceinline__ void con_minmax(int2* p, int32_t x) {
   if (x > c.y) atomicMax(&p->y, x);
 }
 
+// No walk is longer than its tree is deep; the bound ends one over a damaged
+// tree too.
+constexpr int kConWalk = 1 << 22;
+
 // Root of x (its tree complete), with path halving; dead roots are < 0.
 template <class W>
 __device__ __forceinline__ int32_t con_root(int32_t* par, int32_t x) {
   int32_t p = W::ld(par + x);
-  while (p >= 0 && p != x) {
+  for (int it = 0; p >= 0 && p != x && it < kConWalk; ++it) {
     const int32_t q = W::ld(par + p);
     if (q < 0) return q;
     if (q != p) par[x] = q;
@@ -191,14 +204,19 @@ __device__ __forceinline__ int32_t con_root(int32_t* par, int32_t x) {
   }
   return p;
 }
-// Joins the trees of a and b, the larger root under the smaller.
+// Joins the trees of a and b, the larger root under a smaller vertex of the
+// other tree (a root is its tree's smallest id, so a vertex smaller than a
+// root is never below it): only the larger side has to be a root now.
 template <class W>
 __device__ __forceinline__ void con_unite(int32_t* par, int32_t a, int32_t b) {
-  for (;;) {
-    const int32_t ra = con_root<W>(par, a), rb = con_root<W>(par, b);
-    if (ra == rb) return;
-    const int32_t lo = ra < rb ? ra : rb, hi = ra < rb ? rb : ra;
-    if (atomicCAS(par + hi, hi, lo) == hi) return;
+  a = con_root<W>(par, a);
+  b = con_root<W>(par, b);
+  while (a != b) {
+    const int32_t lo = a < b ? a : b, hi = a < b ? b : a;
+    const int32_t p = W::fresh(par + hi);
+    if (p == hi && atomicCAS(par + hi, hi, lo) == hi) return;
+    a = lo;
+    b = p == hi ? W::fresh(par + hi) : p;
   }
 }
 
@@ -242,7 +260,9 @@ __device__ __forceinline__ void con_edges(const Contract& k, const Src& src, con
     src.edges(w, f);
     return;
   }
-  const long long ne = W::ld(k.cntE + t);
+  // (an append past the capacity is counted but not written, and ends the
+  // rounds; the bound keeps even its reader inside the array)
+  const long long ne = min((long long)W::ld(k.cntE + t), k.acap);
   const long long nth = w.threads();
   constexpr int kU = 4;
   for (long long b = w.tid() & ~31ll; b < ne; b += nth * kU) {
@@ -380,11 +400,12 @@ __device__ __noinline__ bool con_round(const Contract& k, const Src& src, const 
 template <class W>
 __device__ __forceinline__ int32_t con_root_at(const Contract& k, int t, int32_t v) {
   const uint32_t h = con_state(t, kConHook), u = con_state(t, kConUnion);
-  for (;;) {
+  for (int it = 0; it < kConWalk; ++it) {
     const uint32_t s = W::ld(k.info + v) & ~kConPos;
-    if (s != h && s != u) return v;
+    if (s != h && s != u) break;
     v = W::ld(k.par + v);
   }
+  return v;
 }
 
 // Undoes round t: the components of the vertices merged in it.
@@ -392,7 +413,8 @@ template <class W>
 __device__ __noinline__ bool con_undo(const Contract& k, const W& w, int t) {
   const long long tid = w.tid(), nth = w.threads();
   const uint32_t stH = con_state(t, kConHook);
-  const int32_t l0 = t > 0 ? W::ld(k.cntL + t) : 0, l1 = W::ld(k.cntL + t + 1);
+  const int32_t l0 = t > 0 ? W::ld(k.cntL + t) : 0;
+  const int32_t l1 = (int32_t)min((long long)W::ld(k.cntL + t + 1), k.lcap);
   const int32_t d0 = t > 0 ? W::ld(k.cntD + t) : 0, d1 = W::ld(k.cntD + t + 1);
   for (long long i = l0 + tid; i < l1; i += nth) {
     const unsigned long long e = W::ld(k.elog + i);
@@ -702,6 +724,36 @@ __device__ __noinline__ void contract_phase(const Args& A, Smem& sm) {
   k.over = &c->con_over;
   Steps st = steps_open(c);
   trace_rec(c, nl, 20);
+  // Vertices that the first round may merge, among one group of 32 in 16:
+  // those with one edge on a side, and those that an out-neighbour points
+  // back to.  Few of either is a uniform random graph, whose core the rounds
+  // do not shrink (with three edges per vertex 29 % have one edge on a side;
+  // on the lattices every vertex counts about once).
+  int may = 0;
+  for (long long j = tid; j < (nl + 15) / 16 + 31; j += nth) {
+    const long long i = (j >> 5) * 512 + (j & 31);
+    if (i >= nl) break;
+    const int32_t v = __ldcg(w.listA + i);
+    const long long s0 = __ldg(g.out.off + v);
+    const long long dout = __ldg(g.out.off + v + 1) - s0;
+    const long long din = __ldg(g.in.off + v + 1) - __ldg(g.in.off + v);
+    if (dout == 1 || din == 1) ++may;
+    bool back = false;
+    for (long long e = s0; e < s0 + dout && e < s0 + kConDegree && !back; ++e) {
+      const int32_t d = __ldg(g.out.adj + e);
+      const long long s1 = __ldg(g.out.off + d), e1 = __ldg(g.out.off + d + 1);
+      for (long long x = s1; x < e1 && x < s1 + kConDegree && !back; ++x)
+        back = d != v && __ldg(g.out.adj + x) == v;
+    }
+    if (back) ++may;
+  }
+  if (may) atomicAdd(&c->con_may, may);
+  if (!step_sync(c, st, 399)) return;
+  // (at most one group of the sample is cut short)
+  if (80ll * __ldcg(&c->con_may) < 2ll * nl) {
+    steps_close(c, st);
+    return;
+  }
   bool big = false;
   for (long long i = tid; i < nl; i += nth) {
     const int32_t v = __ldcg(w.listA + i);
@@ -729,7 +781,7 @@ __device__ __noinline__ void contract_phase(const Args& A, Smem& sm) {
   for (long long i = tid; i < nl; i += nth) {
     const int32_t v = __ldcg(w.listA + i), cv = __ldcg(k.tc + v);
     if (cv < 0) ++open;
-    else if (v < __ldcg(small + cv)) atomicMin(small + cv, v);
+    else if (v < __ldca(small + cv)) atomicMin(small + cv, v);
   }
   for (int o = 16; o; o >>= 1) open += __shfl_xor_sync(kFull, open, o);
   if (lane_id() == 0 && open) atomicAdd(&c->con_open, open);
@@ -738,7 +790,7 @@ __device__ __noinline__ void contract_phase(const Args& A, Smem& sm) {
   for (long long i = tid; i < nl; i += nth) {
     const int32_t v = __ldcg(w.listA + i), cv = __ldcg(k.tc + v);
     if (cv < 0) continue;
-    w.label[v] = __ldcg(small + cv);
+    w.label[v] = __ldca(small + cv);
     if (open) bit_set_red(w.done, v);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) c->ncolour = nl - open;
