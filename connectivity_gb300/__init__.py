@@ -209,8 +209,8 @@ def _take(p: C.c_void_p, count: int, dtype) -> np.ndarray:
 
 
 def _optp(o):
-    """The options argument: o by reference, or NULL (the context's class
-    table, else the defaults)."""
+    """A struct argument by reference, or NULL for None (options: the
+    context's class table, else the defaults; statistics: none wanted)."""
     return C.byref(o) if o is not None else None
 
 
@@ -403,11 +403,12 @@ class Context:
         return out
 
     def _run(self, fn, name, g, labels, o: Opts | None, want_stats: bool):
-        st = Stats()
+        # (statistics cost a pass over the offsets: only when asked for)
+        st = Stats() if want_stats else None
         if labels is None:
             labels = np.empty(g.n, np.int32)
         ptr = _ptr(labels) if isinstance(labels, np.ndarray) else C.c_void_p(int(labels))
-        _check(fn(self._h, g._h, ptr, _optp(o), C.byref(st)), name)
+        _check(fn(self._h, g._h, ptr, _optp(o), _optp(st)), name)
         return (labels, st) if want_stats else labels
 
     def scc(self, g: "Graph", labels=None, o: Opts | None = None, stats: bool = False):
