@@ -97,6 +97,7 @@ struct Ctl {
   // Trim: 16 = start, 17 = degree pass done, 18 = list counted, 19 = list
   // written.  Contraction: 20 = start, 22 / 23 = a round of the
   // grid / of one block, 24 = rounds done, 21 = end.
+  // Residual: 28 = start, 29 = trimmed.
   struct Trace {
     unsigned long long t;
     unsigned long long t_mid;   // pull steps: end of the thread tier
@@ -120,6 +121,9 @@ struct Ctl {
   int32_t con_over;   // an array ran out
   int32_t con_big;    // a vertex has too many edges
   int32_t con_open;   // vertices left without a component
+  int32_t res_cnt[2][2];  // residual: vertices and edges, before and after its trim
+  int32_t res_over;       // an edge list ran out
+  int32_t res_ready;      // its per-vertex state was set by the compaction
   int32_t con_may;    // sampled vertices that the first round may merge
   unsigned long long uf_cross;  // union-find: edges that leave their range
 };

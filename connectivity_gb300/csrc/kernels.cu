@@ -37,11 +37,21 @@ __global__ void k_count_unassigned(Args A) {
   }
 }
 
+// Four labels per thread with their loads together.
 __global__ void k_localize(int32_t* labels, int32_t n, const int32_t* gid, const int64_t* vbase) {
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (long long)gridDim.x * blockDim.x) {
-    const int32_t l = labels[v];
-    if (l >= 0) labels[v] = (int32_t)(l - vbase[gid[v]]);
+  constexpr int kU = 4;
+  const long long nth = (long long)gridDim.x * blockDim.x;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += nth * kU) {
+    int32_t l[kU], g[kU];
+#pragma unroll
+    for (int q = 0; q < kU; ++q) {
+      const bool in = v + q * nth < n;
+      l[q] = in ? labels[v + q * nth] : -1;
+      g[q] = in ? __ldg(gid + v + q * nth) : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kU; ++q)
+      if (l[q] >= 0) labels[v + q * nth] = (int32_t)(l[q] - __ldg(vbase + g[q]));
   }
 }
 
@@ -61,8 +71,8 @@ int max_coop_grid(int device) {
 cudaError_t launch_localize(int32_t* labels, int32_t n, const int32_t* gid, const int64_t* vbase,
                             cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  long long blocks = ((long long)n + 255) / 256;
-  if (blocks > 152 * 16) blocks = 152 * 16;
+  long long blocks = ((long long)n + 1023) / 1024;
+  if (blocks > 152 * 8) blocks = 152 * 8;
   k_localize<<<(int)blocks, 256, 0, s>>>(labels, n, gid, vbase);
   return cudaGetLastError();
 }

@@ -129,42 +129,49 @@ constexpr unsigned kBarrierMaxSpins = 1u << 28;
 
 // Grid-wide barrier for a cooperative launch.  Thread 0 of every block adds
 // one arrival to the barrier word and waits until the arrivals reach the
-// next multiple of the grid size; the word's error bit ends every wait at
-// once.  Every wait is bounded by time and by spin count; on expiry it sets
-// the error.  Returns false when the kernel must stop.
+// grid size times the barriers so far (counted per block; the word starts a
+// run at zero); the word's error bit ends every wait at once.  Every wait is
+// bounded by time and by spin count; on expiry it sets the error.  Returns
+// false when the kernel must stop.
+// The arrival is a reduction with release semantics, so the first poll goes
+// out behind it instead of after its reply, and each poll acquires, so no
+// fence follows: 1.25 us per barrier of 152 blocks that wrote memory, against
+// 1.52 with an atomic that replies and a fence on either side.
 __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ unsigned& bar_epoch() {
+  __shared__ unsigned epoch;  // thread 0 only
+  return epoch;
+}
+// Called by every block before its first barrier.
+__device__ __forceinline__ void bar_open() {
+  if (threadIdx.x == 0) bar_epoch() = 0u;
+}
 __device__ bool grid_barrier(Ctl* c, int where) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned G = gridDim.x;
-    const unsigned long long old = atomicAdd(&c->bar, 1ull);
-    const unsigned arrived = (unsigned)old + 1u;
-    const unsigned target = ((unsigned)old / G + 1u) * G;
-    bool ok = (old & kBarErrBit) == 0ull;
-    if (ok && arrived != target) {
-      const uint64_t t0 = gtimer();
-      unsigned spins = 0;
-      for (;;) {
-        const unsigned long long v = ld_acquire64(&c->bar);
-        if (v & kBarErrBit) { ok = false; break; }
-        if ((int)((unsigned)v - target) >= 0) break;
-        __nanosleep(32);
-        ++spins;
-        if (spins >= kBarrierMaxSpins ||
-            ((spins & 1023u) == 0u && gtimer() - t0 > kBarrierTimeoutNs)) {
-          set_err(c, kErrTimeout, where);
-          ok = false;
-          break;
-        }
+    const unsigned target = bar_epoch() + gridDim.x;
+    bar_epoch() = target;
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&c->bar), "l"(1ull) : "memory");
+    bool ok = true;
+    uint64_t t0 = 0;
+    for (unsigned spins = 0;; ++spins) {
+      const unsigned long long v = ld_acquire64(&c->bar);
+      if (v & kBarErrBit) { ok = false; break; }
+      if ((int)((unsigned)v - target) >= 0) break;
+      __nanosleep(20);
+      if (spins == 0) t0 = gtimer();
+      if (spins >= kBarrierMaxSpins ||
+          ((spins & 1023u) == 1023u && gtimer() - t0 > kBarrierTimeoutNs)) {
+        set_err(c, kErrTimeout, where);
+        ok = false;
+        break;
       }
     }
-    __threadfence();
     s_ok = ok ? 1 : 0;
   }
   __syncthreads();
@@ -680,9 +687,12 @@ __device__ void expand(const int32_t* front, int32_t nfront, const int32_t* heav
   if (t == 0) sm.bl.cnt = 0;
   __syncthreads();
   const long long nw = (long long)G * (T >> 5);
-  // a frontier smaller than 32 per warp is spread over all warps
+  // a frontier smaller than 32 per warp is spread over all warps, one warp of
+  // every block before the next, so that a small one (a batch's pivots, the
+  // last levels of a search) is not left to the first blocks
   const int vpw = (long long)nfront >= nw * 32 ? 32 : (int)(((long long)nfront + nw - 1) / nw);
-  for (long long base = ((long long)b * (T >> 5) + warp) * vpw; base < nfront; base += nw * vpw) {
+  const long long gw = vpw == 32 ? (long long)b * (T >> 5) + warp : (long long)warp * G + b;
+  for (long long base = gw * vpw; base < nfront; base += nw * vpw) {
     const long long i = base + lane;
     int32_t v = -1;
     long long s0 = 0, d0 = 0, s1 = 0, d1 = 0;
@@ -1103,13 +1113,17 @@ struct Args {
   int kind;
 };
 
+struct KeepNothing {
+  __device__ __forceinline__ void operator()(int32_t) const {}
+};
 // Ordered compaction: in[0, nin) -> out, keeping the entries whose bit is
 // clear in `drop`, in list order.  Block b owns a contiguous chunk; one
-// barrier between counting and writing.  The survivor count goes to *total.
-template <class F>
+// barrier between counting and writing.  The survivor count goes to *total;
+// every dropped entry is handed to on_drop, every kept one to on_keep.
+template <class F, class K = KeepNothing>
 __device__ bool compact_ordered(const int32_t* in, int32_t nin, int32_t* out, const uint32_t* drop,
                                 Work& w, Smem& sm, Steps& st, int where, int32_t* total,
-                                Tally& ty, F on_drop) {
+                                Tally& ty, F on_drop, K on_keep = K()) {
   // Every warp owns a contiguous range (ranges follow the global warp
   // order): pass 1 counts what stays and hands every dropped element to
   // on_drop, one grid barrier publishes the block totals, pass 2 writes
@@ -1179,6 +1193,7 @@ __device__ bool compact_ordered(const int32_t* in, int32_t nin, int32_t* out, co
       const unsigned mask = __ballot_sync(kFull, k);
       if (k) {
         out[run + __popc(mask & lanemask_lt())] = v[j];
+        on_keep(v[j]);
         ty.list++;
       }
       run += __popc(mask);
@@ -1350,14 +1365,17 @@ __device__ __forceinline__ void trim_phase(Args& A, Smem& sm) {
             score ? ((score << g.batch.id_bits) | (mask - (unsigned long long)vv)) : 0ull;
         const int32_t gg = (wd < whi && vv < g.n) ? __ldg(g.batch.gid + vv) : -1;
         const int32_t g0 = __shfl_sync(kFull, gg, 0);
+        // (most words hold no key above their graph's best so far)
+        const bool above = key && gg >= 0 && key > __ldcg(g.batch.pkey + gg);
+        if (!__any_sync(kFull, above)) continue;
         if (__all_sync(kFull, gg == g0)) {
           unsigned long long kmax = key;
           for (int o = 16; o; o >>= 1) {
             const unsigned long long k2 = __shfl_xor_sync(kFull, kmax, o);
             kmax = k2 > kmax ? k2 : kmax;
           }
-          if (lane == 0 && kmax && kmax > __ldcg(g.batch.pkey + g0)) atomicMax(g.batch.pkey + g0, kmax);
-        } else if (key && gg >= 0 && key > __ldcg(g.batch.pkey + gg)) {
+          if (lane == 0) atomicMax(g.batch.pkey + g0, kmax);
+        } else if (above) {
           atomicMax(g.batch.pkey + gg, key);
         }
       }
@@ -1581,10 +1599,11 @@ __device__ __forceinline__ void trim_phase(Args& A, Smem& sm) {
       __syncthreads();
     }
   }
-  if (!step_sync(c, st, 5)) return;
-  trace_rec(c, 0, 19);
   // A hint replaces the pivot; level 2 may have trimmed the pivot, in which
   // case FW-BW is skipped and the colour rounds label what is left.
+  // (Thread 0 of block 0 wrote the pivot itself; the bitmap is complete since
+  // the last barrier.  The barrier that ends the phase publishes this, the
+  // list and the step number together.)
   if (b == 0 && t == 0) {
     int32_t pv = c->pivot;
     if (A.p.pivot_hint >= 0 && A.p.pivot_hint < g.n) pv = A.p.pivot_hint;
@@ -1608,6 +1627,7 @@ __device__ __forceinline__ void trim_phase(Args& A, Smem& sm) {
     }
   }
   tally_flush(ty, c, kKTrim, A.p.count_unassigned != 0, sm.red_u);
+  trace_rec(c, 0, 19);
   steps_close(c, st);
 }
 
@@ -1777,12 +1797,20 @@ __device__ void pull_thread(const ReachSpec& R, const Args& A, Work& w, Smem& sm
   const long long nw = (long long)G * (T >> 5);
   const bool hints = R.pull.c[0].hint != nullptr;
   // warps claim runs of candidates from a shared counter, so a warp whose
-  // candidates settle quickly takes more of them; a run is about a quarter
-  // of a warp's even share (between 32 and 2 * kGroup)
+  // candidates settle quickly takes more of them.  A run is one group, whose
+  // loads a lane issues together, or less when there is less than a group
+  // for every warp: a pass over a group costs a chain of dependent loads
+  // whatever it holds.  (Runs of a quarter of a warp's even share made groups
+  // of 256 and 32 on R-MAT-24, the second chain for an eighth of the work, and
+  // of 64 on R-MAT-22: 528 against 520 and 347 against 326 us of device time.)
   constexpr long long kGroup = 32 * kPullA;
   constexpr int kEdgeBatch = 32 * kPullU;
-  long long grab = (long long)ncur / (nw * 4) / 32 * 32;
-  grab = grab < 32 ? 32 : (grab > 2 * kGroup ? 2 * kGroup : grab);
+  const long long share = ((long long)ncur + nw - 1) / nw;
+  const long long turns = (share + kGroup - 1) / kGroup;
+  const long long grab = turns > 0 ? ((share + turns - 1) / turns + 31) / 32 * 32 : 32;
+  // (A first run fixed per warp instead of claimed was slower on R-MAT-24,
+  // 504 -> 540 us of device time: claims hand neighbouring runs to warps that
+  // run at the same time.)
   for (;;) {
     long long clo = 0;
     if (lane == 0)
@@ -2071,8 +2099,13 @@ __device__ bool reach_multi(Search* S, int ns, int* flags /* shared, 2 */, const
     __syncthreads();
     if (flags[0] == 0) break;
     const bool any_pull = flags[1] != 0;
-    for (int k = 0; k < ns; ++k) {
-      const Search& q = S[k];
+    // two pulling searches: every other warp takes the second one's
+    // candidates first, so that the two chains of dependent loads run side by
+    // side (device time of a run: R-MAT-20 261 -> 248 us, R-MAT-22 320 -> 303;
+    // no block barrier lies between them)
+    const bool swap = ns == 2 && S[0].active && S[0].pull && S[1].active && S[1].pull && (warp & 1);
+    for (int j = 0; j < ns; ++j) {
+      const Search& q = S[swap ? 1 - j : j];
       if (!q.active) continue;
       Slot* o = step_out(c, st.s, q.dir);
       if (!q.pull) {
@@ -2381,16 +2414,21 @@ __device__ __forceinline__ void reach_phase(Args& A, Smem& sm) {
   if (batch) {
     for (long long wd = (long long)b * T + t; wd < w.nwords; wd += (long long)G * T) {
       unsigned x = __ldcg(hit + wd);
+      if (x == 0u) continue;
+      // a word inside one graph (most are): its first bit; else the first bit
+      // of every graph in it
+      const int32_t vl = (int32_t)(wd * 32 + 31 - __clz(x));
+      const int32_t gl = __ldg(g.batch.gid + vl);
       int32_t gprev = -1;
       while (x) {
-        const int bit = __ffs(x) - 1;
+        const int32_t v = (int32_t)(wd * 32 + __ffs(x) - 1);
         x &= x - 1;
-        const int32_t v = (int32_t)(wd * 32 + bit);
         const int32_t gg = __ldg(g.batch.gid + v);
         if (gg != gprev) {  // bits rise, so v is the smallest of its graph here
           if (v < __ldcg(g.batch.gmin + gg)) atomicMin(g.batch.gmin + gg, v);
           gprev = gg;
         }
+        if (gg == gl) break;
       }
     }
     if (!step_sync(c, st, 25)) return;
@@ -2417,11 +2455,20 @@ __device__ __forceinline__ void reach_phase(Args& A, Smem& sm) {
     w.label[v] = batch ? (canon ? __ldcg(g.batch.gmin + __ldg(g.batch.gid + v)) : v) : lab;
   };
   trace_rec(c, nvalid, 12);
-  if (!compact_ordered(w.listA, nvalid, w.listB, hit, w, sm, st, 26, &c->nvalid, ty, put)) return;
-  if (!step_sync(c, st, 27)) return;
-  const int32_t nv = __ldcg(&c->nvalid);
-  for (long long i = (long long)b * T + t; i < nv; i += (long long)G * T) w.listA[i] = __ldcg(w.listB + i);
-  trace_rec(c, nv, 15);
+  // (the residual phase starts from these; its lists are free by now)
+  auto stay = [&](int32_t v) {
+    w.live_in[v] = 0;
+    w.live_out[v] = 0x7fffffff;
+  };
+  if (!compact_ordered(w.listA, nvalid, w.listB, hit, w, sm, st, 26, &c->nvalid, ty, put, stay))
+    return;
+  if (b == 0 && t == 0) c->res_ready = 1;
+  // the compacted list takes the valid list's place (published, with its
+  // length, by the barrier that ends the phase)
+  int32_t* const compacted = w.listB;
+  w.listB = w.listA;
+  w.listA = compacted;
+  trace_rec(c, 0, 15);
   tally_flush(ty, c, kKReach, A.p.count_unassigned != 0, sm.red_u);
   steps_close(c, st);
 }

@@ -2,6 +2,7 @@
 // launch, and its launch helpers.
 #pragma once
 #include "run_device.cuh"
+#include "residual_device.cuh"
 
 namespace gb {
 namespace {
@@ -33,6 +34,7 @@ template <int NC, bool kOptions, class Extra = NoExtra>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) k_run(Args A) {
   __shared__ Smem sm;
   sm.stage_base = g_dyn_smem;
+  bar_open();
   Ctl* c = A.w.ctl;
   phase_mark(A, 0);
   trim_phase(A, sm);
@@ -57,9 +59,17 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_run(Args A) {
   // (every block reads the same counts after a barrier, so all take the
   // same branches)
   const bool scc = A.kind == kSCC;
-  if (scc && (A.p.colour_mode == 1 || (A.p.colour_mode == 2 && __ldcg(&c->nvalid) >= kSigMin))) {
+  bool left = true;
+  if constexpr (NC == 1) {
+    if (scc && A.p.colour_mode == 2) {
+      left = residual_phase(A, sm);
+      if (left && !grid_barrier(c, 905)) return;
+    }
+  }
+  if (left && scc &&
+      (A.p.colour_mode == 1 || (A.p.colour_mode == 2 && __ldcg(&c->nvalid) >= kSigMin))) {
     signature_rounds(A, sm, A.w.listA, A.w.listB);
-  } else {
+  } else if (left) {
     // colour_mode 2: a residual still left after kSigAfter colour rounds
     // goes on in signature rounds (a deep condensation: chains)
     const int cap = scc && A.p.colour_mode == 2 ? kSigAfter : 0x7fffffff;
