@@ -1239,8 +1239,18 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
     return s;
   }
   cudaStream_t sm = c->stream;
-  const bool dev_edges = m == 0 || is_device_ptr(src);
+  bool dev_edges = m == 0 || is_device_ptr(src);
   const bool dev_labels = is_device_ptr(labels);
+  // a short list in host memory that the device reads is used in place: two
+  // copies cost more than the block's reads over the host link
+  if (small && !dev_edges && m <= gb::kSmallAutoEdges) {
+    const void *vs = host_view(src), *vd = host_view(dst);
+    if (vs && vd) {
+      src = (const int32_t*)vs;
+      dst = (const int32_t*)vd;
+      dev_edges = true;
+    }
+  }
   // one stream-ordered allocation: the edges (from host memory), the SCC
   // CSR built by the block (2m ints) and the labels (for host labels)
   const size_t edge_b = dev_edges ? 0 : (size_t)m * 8;

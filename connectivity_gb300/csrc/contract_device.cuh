@@ -103,8 +103,7 @@ struct ConGrid {
 };
 struct ConBlock {
   static constexpr bool kStaged = false;
-  Ctl* c;
-  volatile int* left;  // shared: steps this block may still take
+  volatile int* left;  // shared: steps this block may still take, < 0: too many
   __device__ __forceinline__ long long tid() const { return threadIdx.x; }
   __device__ __forceinline__ long long threads() const { return blockDim.x; }
   template <class T>
@@ -115,9 +114,9 @@ struct ConBlock {
     const volatile int* q = reinterpret_cast<const volatile int*>(p);
     return make_int2(q[0], q[1]);
   }
-  __device__ __forceinline__ bool sync(int where) const {
+  __device__ __forceinline__ bool sync(int) const {
     __syncthreads();
-    if (threadIdx.x == 0 && --*left < 0) set_err(c, kErrIterLimit, where);
+    if (threadIdx.x == 0) --*left;
     __syncthreads();
     return *left >= 0;
   }
@@ -537,33 +536,33 @@ __device__ __forceinline__ bool con_core(const Contract& k, const W& w, int t, v
   }
 }
 
-// The tail: block 0 finishes the graph of round t in its shared memory
-// (n0 <= kConTailVerts, E_t <= kConTailEdges) and leaves a component in tc
-// for every vertex of A_t.
-constexpr int32_t kConTailBytes =
-    kConTailVerts * 44 + (2 * kConTailEdges + kConTailLog) * 8;
-static_assert(kConTailBytes <= kDynSmem, "the tail's arrays fit the dynamic shared memory");
-__device__ __noinline__ void con_tail(const Contract& k, Ctl* c, int t, int32_t steps_left,
-                                      int32_t* smem, int32_t* rounds) {
-  __shared__ int s_left, s_flag;
+// One block's contraction of a graph of n <= V vertices (ids 0 to n - 1) in
+// con_bytes(V, E, L) bytes of its shared memory; src enumerates the edges, at
+// most E; L entries of log.  Afterwards comp[i] (in smem, valid until it is reused)
+// is the component of vertex i, the id of one of its members, or kConOpen
+// when the log ran out.  *left: steps the block may still take; negative
+// afterwards when they ran out (comp is then not set).  Returns the rounds.
+constexpr int32_t con_bytes(int32_t V, int32_t E, int32_t L) { return V * 40 + (2 * E + L) * 8; }
+template <int32_t V, int32_t E, int32_t L, class Src>
+__device__ __noinline__ int con_solve(const Src& src, int32_t n, int32_t* smem,
+                                      volatile int* left, int32_t** comp) {
+  __shared__ int s_flag;
   __shared__ int32_t s_cnt[4][kConRounds + 2];
   __shared__ int32_t s_over;
   const int tid = threadIdx.x, nth = blockDim.x;
-  const int32_t n = __ldcg(k.cntA + t);
   Contract l;
   l.arena = reinterpret_cast<unsigned long long*>(smem);
-  l.acap = 2 * kConTailEdges;  // E_u and E_{u+1} always fit
-  l.elog = l.arena + 2 * kConTailEdges;
-  l.lcap = kConTailLog;
-  l.in = reinterpret_cast<int2*>(l.elog + kConTailLog);
-  l.out = l.in + kConTailVerts;
-  l.par = reinterpret_cast<int32_t*>(l.out + kConTailVerts);
-  l.tc = l.par + kConTailVerts;
-  l.info = reinterpret_cast<uint32_t*>(l.tc + kConTailVerts);
-  l.A[0] = l.tc + 2 * kConTailVerts;
-  l.A[1] = l.A[0] + kConTailVerts;
-  l.D = l.A[1] + kConTailVerts;
-  int32_t* const gid = l.D + kConTailVerts;
+  l.acap = 2 * E;  // E_u and E_{u+1} always fit
+  l.elog = l.arena + 2 * E;
+  l.lcap = L;
+  l.in = reinterpret_cast<int2*>(l.elog + L);
+  l.out = l.in + V;
+  l.par = reinterpret_cast<int32_t*>(l.out + V);
+  l.tc = l.par + V;
+  l.info = reinterpret_cast<uint32_t*>(l.tc + V);
+  l.A[0] = l.tc + 2 * V;
+  l.A[1] = l.A[0] + V;
+  l.D = l.A[1] + V;
   l.list0 = nullptr;
   l.n0 = n;
   l.cntA = s_cnt[0];
@@ -571,23 +570,17 @@ __device__ __noinline__ void con_tail(const Contract& k, Ctl* c, int t, int32_t 
   l.cntD = s_cnt[2];
   l.cntL = s_cnt[3];
   l.over = &s_over;
-  if (tid == 0) {
-    s_left = steps_left;
-    s_over = 0;
-  }
+  *comp = l.tc;
+  if (tid == 0) s_over = 0;
   for (int i = tid; i < 4 * (kConRounds + 2); i += nth) (&s_cnt[0][0])[i] = 0;
   for (int i = tid; i < n; i += nth) {
-    const int32_t v = __ldcg(k.A[t & 1] + i);
-    gid[i] = v;
-    k.tc[v] = i;
     l.in[i] = make_int2(kConInf, -1);
     l.out[i] = make_int2(kConInf, -1);
     l.par[i] = i;
     l.info[i] = 0u;
   }
   __syncthreads();
-  const ConBlock b{c, &s_left};
-  const ConLocal src{&k, t};
+  const ConBlock b{left};
   int u = 0;
   bool ok = true;
   for (;;) {
@@ -607,8 +600,35 @@ __device__ __noinline__ void con_tail(const Contract& k, Ctl* c, int t, int32_t 
   }
   __syncthreads();
   for (int x = u - (undone ? 2 : 1); ok && x >= 0; --x) ok = con_undo(l, b, x);
+  return u;
+}
+
+// The tail: block 0 finishes the graph of round t (at most kConTailVerts
+// vertices and kConTailEdges edges) and leaves a component in tc for every
+// vertex of A_t.
+constexpr int32_t kConTailBytes = con_bytes(kConTailVerts, kConTailEdges, kConTailLog);
+static_assert(kConTailBytes + kConTailVerts * 4 <= kDynSmem,
+              "the tail's arrays fit the dynamic shared memory");
+__device__ __forceinline__ void con_tail(const Contract& k, Ctl* c, int t, int32_t steps_left,
+                                         int32_t* smem, int32_t* rounds) {
+  __shared__ int s_left;
+  int32_t* const gid = smem + kConTailBytes / 4;
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const int32_t n = __ldcg(k.cntA + t);
+  if (tid == 0) s_left = steps_left;
   for (int i = tid; i < n; i += nth) {
-    const int32_t x = ok ? l.tc[i] : kConOpen;
+    const int32_t v = __ldcg(k.A[t & 1] + i);
+    gid[i] = v;
+    k.tc[v] = i;
+  }
+  __syncthreads();
+  int32_t* comp;
+  const int u = con_solve<kConTailVerts, kConTailEdges, kConTailLog>(ConLocal{&k, t}, n, smem,
+                                                                     &s_left, &comp);
+  const bool ok = s_left >= 0;
+  if (!ok && tid == 0) set_err(c, kErrIterLimit, 431);
+  for (int i = tid; i < n; i += nth) {
+    const int32_t x = ok ? comp[i] : kConOpen;
     k.tc[gid[i]] = x < 0 ? kConOpen : gid[x];
   }
   if (tid == 0) *rounds = t + u;

@@ -285,8 +285,9 @@ struct SmallDesc {
   int32_t* adj_scratch;
   int32_t* labels;          // n outputs: smallest member id per component
 };
-// Dynamic shared memory of a block for graphs of at most max_n vertices.
-size_t small_smem_bytes(int32_t max_n);
+// Dynamic shared memory of a block for graphs of at most max_n vertices
+// (kind as for launch_small).
+size_t small_smem_bytes(int kind, int32_t max_n);
 // kind 0 = SCC, 1 = WCC.  One block per graph: `count` descriptors from
 // `many` (device memory), or `one` when many is null (count 1).  A failure
 // (an id outside [0, n) in edge form: kErrInvalid; a loop past max_steps:

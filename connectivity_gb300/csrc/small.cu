@@ -23,11 +23,14 @@
 //      after four of them, signature rounds until no vertex is left (the
 //      smallest reaching and reached ids inside classes of equal pairs;
 //      equal ids label the vertex).
+// Under colour_mode 2, graphs with a hub take a shorter way to the same labels
+// (hub_scc): two searches from the hub together, then a contraction of what
+// they leave; R-MAT of 4,000 vertices and 52,000 edges: 178 -> 60 us a call.
 // WCC (cc_main.cpp:184-245): union-find over the edges with hooking of the
 // larger root under the smaller, so each root is its component's smallest
 // id; no fixed-point loop.
 //
-// Frontier steps are edge-balanced: the frontier's degrees are scanned, and
+// Frontier steps of the general way are edge-balanced: the frontier's degrees are scanned, and
 // thread t takes edges t, t + 1024, ... of the concatenated edge lists,
 // finding its vertex by a binary search over the scan, so a hub's edges are
 // spread over the whole block.
@@ -37,7 +40,7 @@
 // scattered here into a caller-provided scratch area (2m ints).
 #include <cstdint>
 
-#include "gb_internal.cuh"
+#include "contract_device.cuh"
 
 namespace gb {
 namespace {
@@ -51,6 +54,7 @@ constexpr int kCtlInts = 160;
 constexpr int cQn = 0;       // queue lengths [2]
 constexpr int cBad = 2;      // an edge id outside [0, n)
 constexpr int cStop = 3;     // a loop ran out of steps
+constexpr int cLeft = 4;     // steps the contraction of a rest may take
 constexpr int cRed = 8;      // reductions: up to 3 * kSW words
 constexpr int cScan = 112;   // scans: kSW + 1 words
 
@@ -151,6 +155,35 @@ struct SmallCsr {
   int32_t base;         // subtracted from every adjacency entry
 };
 
+// The block's shared memory for n vertices, derived in every function from
+// the array itself, so that accesses are known to be to shared memory.
+struct SmallMem {
+  int32_t* ctl;
+  int32_t* ooff;   // n + 1
+  int32_t* ioff;   // n + 1
+  int32_t* lab;    // n from here on
+  uint32_t* flg;
+  int32_t* cnt_o;
+  int32_t* cnt_i;
+  int32_t* q[2];
+  int32_t* pre;    // n + 1
+};
+extern __shared__ __align__(16) int32_t g_small_smem[];
+__device__ __forceinline__ SmallMem small_mem(int n) {
+  SmallMem s;
+  s.ctl = g_small_smem;
+  s.ooff = g_small_smem + kCtlInts;
+  s.ioff = s.ooff + (n + 1);
+  s.lab = s.ioff + (n + 1);
+  s.flg = reinterpret_cast<uint32_t*>(s.lab + n);
+  s.cnt_o = s.lab + 2 * n;
+  s.cnt_i = s.cnt_o + n;
+  s.q[0] = s.cnt_i + n;
+  s.q[1] = s.cnt_i + 2 * n;
+  s.pre = s.cnt_i + 3 * n;
+  return s;
+}
+
 // Visits every edge (v, w) of the frontier's adjacency lists, edge-balanced.
 // pre: n + 1 ints of scratch.  Ends with a barrier.
 template <class F>
@@ -190,6 +223,25 @@ __device__ void for_each_edge(int n, const int32_t* off, const int32_t* adj, int
   }
 }
 
+// Every edge (a, b) of a list, eight per thread with their loads together
+// (the list may be in host memory, read over the host link).
+template <class F>
+__device__ void for_each_listed(const SmallDesc& D, F f) {
+  constexpr int kU = 8;
+  for (long long e0 = threadIdx.x; e0 < D.m; e0 += kST * kU) {
+    int32_t a[kU], b[kU];
+#pragma unroll
+    for (int q = 0; q < kU; ++q) {
+      const bool in = e0 + q * kST < D.m;
+      a[q] = in ? D.src[e0 + q * kST] - D.id_base : 0;
+      b[q] = in ? D.dst[e0 + q * kST] - D.id_base : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kU; ++q)
+      if (e0 + q * kST < D.m) f(a[q], b[q]);
+  }
+}
+
 __device__ __forceinline__ void push(int32_t* q, int32_t* qn, int32_t v) {
   q[atomicAdd(qn, 1)] = v;
 }
@@ -216,125 +268,249 @@ __device__ __forceinline__ void uf_unite(int32_t* p, int32_t a, int32_t b) {
   }
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc* many,
-                                                  int32_t max_steps, int32_t colour_rounds,
-                                                  int* err) {
-  extern __shared__ int32_t smem[];
-  const SmallDesc D = many ? many[blockIdx.x] : one;
-  const int n = D.n;
-  if (n <= 0) return;
-  const int tid = threadIdx.x;
-  int32_t* ctl = smem;
-  int32_t* ooff = smem + kCtlInts;
-  int32_t* ioff = ooff + (n + 1);
-  int32_t* lab = ioff + (n + 1);
-  uint32_t* flg = reinterpret_cast<uint32_t*>(lab + n);
-  int32_t* cnt_o = reinterpret_cast<int32_t*>(flg + n);
-  int32_t* cnt_i = cnt_o + n;
-  int32_t* q[2] = {cnt_i + n, cnt_i + 2 * n};
-  int32_t* pre = cnt_i + 3 * n;  // n + 1
+// ---- graphs with a hub ------------------------------------------------------
+// A pivot of at least kHubDeg edges on both sides: the graph's large component
+// lies within a few hops of it, and most vertices have a neighbour that is
+// reached early.  Then, instead of the trim to the fixed point, the frontier
+// queues and the colour rounds (a binary search and a chain of L2 loads per
+// edge: 156 us for 4,000 vertices and 52,000 edges):
+//   - both searches advance in the same passes, from below: a vertex that is
+//     not reached looks through its list until it finds one that is;
+//   - the edges between the vertices left are listed, and those without both
+//     an in- and an out-edge among them labelled;
+//   - what remains is contracted (con_solve).
+// A rest too large for the contraction goes to the colour rounds.
+constexpr int32_t kHubDeg = 16;
+constexpr int32_t kSigAfterSmall = 4;  // colour rounds of colour_mode 2
+
+// One pass of a search from below for vertex v of this lane (valid and not
+// reached when `need`): whether a neighbour in adj[s, s + d) is reached
+// (`bit`).  Eight entries by the lane, the rest by the warp.  All lanes call.
+__device__ __forceinline__ bool hub_look(const uint32_t* flg, const int32_t* adj, int32_t base,
+                                         uint32_t bit, bool need, int32_t s, int32_t d) {
+  bool hit = false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    int32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w[q] = need && !hit && 4 * h + q < d ? adj[s + 4 * h + q] - base : -1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) hit = hit || (w[q] >= 0 && (flg[w[q]] & bit));
+  }
+  unsigned more = __ballot_sync(kFull, need && !hit && d > 8);
+  const int lane = threadIdx.x & 31;
+  while (more) {
+    const int j = __ffs(more) - 1;
+    more &= more - 1;
+    const int32_t sj = __shfl_sync(kFull, s, j), dj = __shfl_sync(kFull, d, j);
+    bool any = false;
+    for (int32_t e = 8; e < dj && !any; e += 128) {
+      bool h = false;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int32_t i = e + 32 * q + lane;
+        const int32_t w = i < dj ? adj[sj + i] - base : -1;
+        h = h || (w >= 0 && (flg[w] & bit));
+      }
+      any = __any_sync(kFull, h);
+    }
+    if (lane == j) hit = hit || any;
+  }
+  return hit;
+}
+
+// Edges of the residual between local ids (loc).
+struct HubRest {
+  const uint32_t* e;
+  int n;
+  const int32_t* loc;
+  template <class W, class F>
+  __device__ __forceinline__ void edges(const W& w, F f) const {
+    for (int b = (int)w.tid() & ~31; b < n; b += (int)w.threads()) {
+      const int i = b + (int)(threadIdx.x & 31);
+      const uint32_t x = i < n ? e[i] : 0u;
+      f(i < n ? loc[x >> 16] : 0, i < n ? loc[x & 0xffffu] : 0, i < n);
+    }
+  }
+};
+
+// SCC of a graph with a hub, up to the vertices that con_solve could not take:
+// their number is returned, their flg is kValid, every other vertex has its
+// label in lab.  Uses kHubSmem bytes of shared memory past the flags.
+// (R-MAT graphs leave a few dozen vertices.  Room for 1,024 took enough from
+// the L1 to slow the general path by 7 %, which reads its lists through it.)
+constexpr int32_t kHubVerts = 512, kHubEdges = 1536, kHubLog = 1280;
+constexpr int32_t kHubCon = con_bytes(kHubVerts, kHubEdges, kHubLog);
+constexpr int32_t kHubSmem = kHubCon + kHubVerts * 4 + kHubEdges * 4;
+__device__ __noinline__ int32_t hub_scc(int n, int32_t pivot, const int32_t* oadj,
+                                        const int32_t* iadj, int32_t base, int32_t cap) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const SmallMem s = small_mem(n);
+  const int32_t* const ooff = s.ooff;
+  const int32_t* const ioff = s.ioff;
+  int32_t* const lab = s.lab;
+  uint32_t* const flg = s.flg;
+  int32_t* const ctl = s.ctl;
+  // (16-byte aligned, after the flags)
+  int32_t* const tail = g_small_smem + ((kCtlInts + 4 * n + 2 + 3) & ~3);
   int32_t* qn = ctl + cQn;
-  const int32_t cap = (int32_t)min((long long)max_steps, 4ll * n + 64);
+  // valid: an edge on either side; the pivot's neighbours are reached
+  for (int v = tid; v < n; v += kST) {
+    const bool valid = ooff[v + 1] > ooff[v] && ioff[v + 1] > ioff[v];
+    flg[v] = valid ? kValid : 0u;
+    lab[v] = valid ? -1 : v;
+  }
+  __syncthreads();
+  for (int e = ooff[pivot] + tid; e < ooff[pivot + 1]; e += kST)
+    atomicOr(&flg[oadj[e] - base], kFw);
+  for (int e = ioff[pivot] + tid; e < ioff[pivot + 1]; e += kST)
+    atomicOr(&flg[iadj[e] - base], kBw);
+  if (tid == 0) atomicOr(&flg[pivot], kFw | kBw);
+  int32_t pass = 0;
+  for (bool open = true; open; ++pass) {
+    if (pass >= cap) {
+      ctl[cStop] = 1;
+      return 0;
+    }
+    __syncthreads();
+    if (tid == 0) qn[0] = 0;
+    __syncthreads();
+    bool grew = false;
+    for (int v0 = tid & ~31; v0 < n; v0 += kST) {
+      const int v = v0 + lane;
+      const uint32_t f = v < n ? flg[v] : 0u;
+      const bool nf = (f & (kValid | kFw)) == kValid, nb = (f & (kValid | kBw)) == kValid;
+      const int32_t is = nf ? ioff[v] : 0, id = nf ? ioff[v + 1] - is : 0;
+      const int32_t os = nb ? ooff[v] : 0, od = nb ? ooff[v + 1] - os : 0;
+      const bool hf = hub_look(flg, iadj, base, kFw, nf, is, id);
+      const bool hb = hub_look(flg, oadj, base, kBw, nb, os, od);
+      if (hf || hb) {
+        flg[v] = f | (hf ? kFw : 0u) | (hb ? kBw : 0u);  // (only this lane writes it)
+        grew = true;
+      }
+    }
+    if (__any_sync(kFull, grew) && lane == 0) qn[0] = 1;
+    __syncthreads();
+    open = qn[0] != 0;
+  }
+  // the component takes its smallest member; the rest is listed
+  int32_t mn = 0x7fffffff;
+  for (int v = tid; v < n; v += kST)
+    if ((flg[v] & (kValid | kFw | kBw)) == (kValid | kFw | kBw)) mn = min(mn, v);
+  mn = block_min(mn, ctl);
+  if (tid == 0) qn[0] = qn[1] = 0;
+  int32_t left = 0;
+  for (int v = tid; v < n; v += kST) {
+    const uint32_t f = flg[v];
+    if (!(f & kValid)) {
+      flg[v] = 0;
+    } else if ((f & (kFw | kBw)) == (kFw | kBw)) {
+      lab[v] = mn;
+      flg[v] = 0;
+    } else {
+      flg[v] = kValid;
+      ++left;
+    }
+  }
+  left = block_sum(left, ctl);
+  if (left == 0) return 0;
+  int32_t* const rest = tail + kHubCon / 4;
+  uint32_t* const edges = reinterpret_cast<uint32_t*>(rest + kHubVerts);
+  // edges between the vertices left, a warp per vertex; kFw: has an out-edge,
+  // kBw: has an in-edge
+  for (int v = tid >> 5; v < n; v += kSW) {
+    if (!(flg[v] & kValid)) continue;
+    for (int32_t e = ooff[v] + lane; e < ooff[v + 1]; e += 32) {
+      const int32_t w = oadj[e] - base;
+      if (w == v || !(flg[w] & kValid)) continue;
+      atomicOr(&flg[v], kFw);
+      atomicOr(&flg[w], kBw);
+      const int at = atomicAdd(&qn[1], 1);
+      if (at < kHubEdges) edges[at] = ((uint32_t)v << 16) | (uint32_t)w;
+    }
+  }
+  __syncthreads();
+  left = 0;
+  for (int v = tid; v < n; v += kST) {
+    const uint32_t f = flg[v];
+    if (!(f & kValid)) continue;
+    if ((f & (kFw | kBw)) == (kFw | kBw)) {
+      flg[v] = kValid;
+      const int at = atomicAdd(&qn[0], 1);
+      if (at < kHubVerts) {
+        rest[at] = v;
+        lab[v] = at;  // its local id until it is labelled
+      }
+      ++left;
+    } else {
+      lab[v] = v;
+      flg[v] = 0;
+    }
+  }
+  left = block_sum(left, ctl);
+  const int ne = qn[1];
+  if (left == 0 || left > kHubVerts || ne > kHubEdges) return left;
+  __syncthreads();
   if (tid == 0) {
-    ctl[cBad] = 0;
-    ctl[cStop] = 0;
+    qn[1] = 0;
+    ctl[cLeft] = cap - pass;
   }
-
-  // ---- WCC from an edge list: union-find over the edges, no CSR ----------
-  if (KIND == 1 && D.out_off == nullptr) {
-    for (int v = tid; v < n; v += kST) lab[v] = v;
+  // edges of vertices labelled just now drop out, a stretch of the block at a
+  // time (what is kept never passes what is read)
+  for (int b0 = 0; b0 < ne; b0 += kST) {
+    const int i = b0 + tid;
+    const uint32_t x = i < ne ? edges[i] : 0u;
+    const bool keep = i < ne && (flg[x >> 16] & kValid) && (flg[x & 0xffffu] & kValid);
     __syncthreads();
-    for (long long e = tid; e < D.m; e += kST) {
-      const int32_t a = D.src[e] - D.id_base, b = D.dst[e] - D.id_base;
-      if ((unsigned)a >= (unsigned)n || (unsigned)b >= (unsigned)n) {
-        ctl[cBad] = 1;
-        continue;
-      }
-      uf_unite(lab, a, b);
-    }
+    if (keep) edges[atomicAdd(&qn[1], 1)] = x;
     __syncthreads();
-    if (ctl[cBad]) {
-      if (tid == 0) atomicCAS(err, 0, (int)kErrInvalid);
-      return;
-    }
-    for (int v = tid; v < n; v += kST) D.labels[v] = uf_find(lab, v);
-    return;
   }
-
-  // ---- the CSR ------------------------------------------------------------
-  SmallCsr g;
-  if (D.out_off != nullptr) {
-    const long long ob = D.out_off[0];
-    const long long ib = D.in_off ? D.in_off[0] : ob;
-    for (int v = tid; v <= n; v += kST) {
-      ooff[v] = (int32_t)(D.out_off[v] - ob);
-      ioff[v] = D.in_off ? (int32_t)(D.in_off[v] - ib) : ooff[v];
-    }
-    g.oadj = D.out_adj + ob;
-    g.iadj = D.in_off ? D.in_adj + ib : g.oadj;
-    g.base = D.id_base;
-  } else {
-    for (int v = tid; v < n; v += kST) {
-      cnt_o[v] = 0;
-      cnt_i[v] = 0;
-    }
-    __syncthreads();
-    for (long long e = tid; e < D.m; e += kST) {
-      const int32_t a = D.src[e] - D.id_base, b = D.dst[e] - D.id_base;
-      if ((unsigned)a >= (unsigned)n || (unsigned)b >= (unsigned)n) {
-        ctl[cBad] = 1;
-        continue;
-      }
-      atomicAdd(&cnt_o[a], 1);
-      atomicAdd(&cnt_i[b], 1);
-    }
-    __syncthreads();
-    if (ctl[cBad]) {
-      if (tid == 0) atomicCAS(err, 0, (int)kErrInvalid);
-      return;
-    }
-    for (int v = tid; v < n; v += kST) {
-      ooff[v] = cnt_o[v];
-      ioff[v] = cnt_i[v];
-    }
-    if (tid == 0) {
-      ooff[n] = 0;
-      ioff[n] = 0;
-    }
-    block_scan(ooff, n + 1, ctl);
-    block_scan(ioff, n + 1, ctl);
-    for (int v = tid; v < n; v += kST) {
-      cnt_o[v] = ooff[v];
-      cnt_i[v] = ioff[v];
-    }
-    __syncthreads();
-    int32_t* so = D.adj_scratch;
-    int32_t* si = D.adj_scratch + D.m;
-    for (long long e = tid; e < D.m; e += kST) {
-      const int32_t a = D.src[e] - D.id_base, b = D.dst[e] - D.id_base;
-      so[atomicAdd(&cnt_o[a], 1)] = b;
-      si[atomicAdd(&cnt_i[b], 1)] = a;
-    }
-    __syncthreads();
-    g.oadj = so;
-    g.iadj = si;
-    g.base = 0;
+  __syncthreads();
+  int32_t* comp;
+  con_solve<kHubVerts, kHubEdges, kHubLog>(HubRest{edges, qn[1], lab}, left, tail, ctl + cLeft,
+                                           &comp);
+  __syncthreads();
+  if (ctl[cLeft] < 0) {
+    ctl[cStop] = 1;
+    return 0;
   }
-  g.ooff = ooff;
-  g.ioff = ioff;
-
-  // ---- WCC on a CSR: union-find over the out-lists ------------------------
-  if (KIND == 1) {
-    for (int v = tid; v < n; v += kST) lab[v] = v;
-    __syncthreads();
-    for_each_edge(n, ooff, g.oadj, g.base, [&](int32_t u, int32_t w) { uf_unite(lab, u, w); });
-    __syncthreads();
-    for (int v = tid; v < n; v += kST) D.labels[v] = uf_find(lab, v);
-    return;
+  int32_t* const small = tail;  // (the contraction's edges are done with)
+  for (int i = tid; i < left; i += kST) small[i] = 0x7fffffff;
+  __syncthreads();
+  for (int i = tid; i < left; i += kST)
+    if (comp[i] >= 0) atomicMin(&small[comp[i]], rest[i]);
+  __syncthreads();
+  int32_t open = 0;
+  for (int i = tid; i < left; i += kST) {
+    const int32_t v = rest[i];
+    lab[v] = comp[i] >= 0 ? small[comp[i]] : -1;
+    if (comp[i] >= 0) flg[v] = 0;
+    else ++open;
   }
+  return block_sum(open, ctl);
+}
 
-  // ---- SCC ----------------------------------------------------------------
+// The general path: trim to the fixed point, FW-BW, colour and signature
+// rounds by frontier queues.  nvalid >= 0: only the rounds, for the vertices
+// that hub_scc left.  (Not inlined, as hub_scc is not: with both in the kernel
+// the registers kept across their calls made this path 8 % slower.)
+__device__ __noinline__ void queue_scc(int n, const int32_t* oadj, const int32_t* iadj,
+                                       int32_t base, int32_t cap, int32_t colour_rounds,
+                                       int32_t nvalid) {
+  const int tid = threadIdx.x;
+  const SmallMem s = small_mem(n);
+  int32_t* const ctl = s.ctl;
+  int32_t* const ooff = s.ooff;
+  int32_t* const ioff = s.ioff;
+  int32_t* const lab = s.lab;
+  uint32_t* const flg = s.flg;
+  int32_t* const cnt_o = s.cnt_o;
+  int32_t* const cnt_i = s.cnt_i;
+  int32_t* const q[2] = {s.q[0], s.q[1]};
+  int32_t* const pre = s.pre;
+  int32_t* const qn = ctl + cQn;
+  int cur = 0;
+  if (nvalid < 0) {
   // live degrees without self-loops
   for (int v = tid; v < n; v += kST) {
     cnt_o[v] = ooff[v + 1] - ooff[v];
@@ -343,7 +519,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
     lab[v] = -1;
   }
   __syncthreads();
-  for_each_edge(n, ooff, g.oadj, g.base, [&](int32_t u, int32_t w) {
+  for_each_edge(n, ooff, oadj, base, [&](int32_t u, int32_t w) {
     if (u == w) {
       atomicSub(&cnt_o[u], 1);
       atomicSub(&cnt_i[u], 1);
@@ -368,7 +544,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
       push(q[nx], &qn[nx], w);
     }
   };
-  int cur = 0;
+  cur = 0;
   for (int32_t it = 0;; ++it) {
     const int nf = qn[cur];
     if (nf == 0) break;
@@ -379,10 +555,10 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
     const int nx = cur ^ 1;
     if (tid == 0) qn[nx] = 0;
     __syncthreads();
-    expand_front(q[cur], nf, ooff, g.oadj, g.base, pre, ctl, [&](int32_t v, int32_t w) {
+    expand_front(q[cur], nf, ooff, oadj, base, pre, ctl, [&](int32_t v, int32_t w) {
       if (w != v && (flg[w] & kValid) && atomicSub(&cnt_i[w], 1) == 1) claim_trim(w, nx);
     });
-    expand_front(q[cur], nf, ioff, g.iadj, g.base, pre, ctl, [&](int32_t v, int32_t w) {
+    expand_front(q[cur], nf, ioff, iadj, base, pre, ctl, [&](int32_t v, int32_t w) {
       if (w != v && (flg[w] & kValid) && atomicSub(&cnt_o[w], 1) == 1) claim_trim(w, nx);
     });
     cur = nx;
@@ -390,7 +566,6 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
   __syncthreads();
 
   // 2. FW-BW from the pivot
-  int32_t nvalid;
   {
     long long key = -1;
     int32_t id = 0x7fffffff;
@@ -413,7 +588,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
         }
         __syncthreads();
         const int32_t* off = dir == 0 ? ooff : ioff;
-        const int32_t* adj = dir == 0 ? g.oadj : g.iadj;
+        const int32_t* adj = dir == 0 ? oadj : iadj;
         const uint32_t want = dir == 0 ? kValid : (kValid | kFw);
         const uint32_t mask = dir == 0 ? (kValid | kFw) : (kValid | kFw | kBw);
         const uint32_t bit = dir == 0 ? kFw : kBw;
@@ -428,7 +603,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
           const int nx = cur ^ 1;
           if (tid == 0) qn[nx] = 0;
           __syncthreads();
-          expand_front(q[cur], nf, off, adj, g.base, pre, ctl, [&](int32_t v, int32_t w) {
+          expand_front(q[cur], nf, off, adj, base, pre, ctl, [&](int32_t v, int32_t w) {
             if ((flg[w] & mask) == want && !(atomicOr(&flg[w], bit) & bit))
               push(q[nx], &qn[nx], w);
           });
@@ -455,6 +630,8 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
       nvalid -= block_sum(cnt2, ctl);
     }
   }
+  }
+  __syncthreads();
 
   // 3. colour rounds (at most colour_rounds), then signature rounds for what
   // is left
@@ -488,7 +665,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
       if (tid == 0) qn[nx] = 0;
       for (int i = tid; i < nf; i += kST) atomicAnd(&flg[q[cur][i]], ~kInq);
       __syncthreads();
-      expand_front(q[cur], nf, ooff, g.oadj, g.base, pre, ctl, [&](int32_t v, int32_t w) {
+      expand_front(q[cur], nf, ooff, oadj, base, pre, ctl, [&](int32_t v, int32_t w) {
         if (!(flg[w] & kValid)) return;
         const int32_t cv = col[v];
         if (col[w] > cv && atomicMin(&col[w], cv) > cv && !(atomicOr(&flg[w], kInq) & kInq))
@@ -518,7 +695,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
       const int nx = cur ^ 1;
       if (tid == 0) qn[nx] = 0;
       __syncthreads();
-      expand_front(q[cur], nf, ioff, g.iadj, g.base, pre, ctl, [&](int32_t v, int32_t w) {
+      expand_front(q[cur], nf, ioff, iadj, base, pre, ctl, [&](int32_t v, int32_t w) {
         if ((flg[w] & (kValid | kFw)) == kValid && col[w] == col[v] &&
             !(atomicOr(&flg[w], kFw) & kFw))
           push(q[nx], &qn[nx], w);
@@ -570,7 +747,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
         if (tid == 0) qn[nx] = 0;
         for (int i = tid; i < nf; i += kST) atomicAnd(&flg[q[cur][i]], ~kInq);
         __syncthreads();
-        expand_front(q[cur], nf, off, adj, g.base, pre, ctl, [&](int32_t v, int32_t w) {
+        expand_front(q[cur], nf, off, adj, base, pre, ctl, [&](int32_t v, int32_t w) {
           if (!(flg[w] & kValid) || lab[w] != lab[v]) return;
           const int32_t cv = val[v];
           if (val[w] > cv && atomicMin(&val[w], cv) > cv && !(atomicOr(&flg[w], kInq) & kInq))
@@ -584,9 +761,9 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
         ctl[cStop] = 1;
         break;
       }
-      propagate(fw, ooff, g.oadj);
+      propagate(fw, ooff, oadj);
       if (ctl[cStop]) break;
-      propagate(bw, ioff, g.iadj);
+      propagate(bw, ioff, iadj);
       if (ctl[cStop]) break;
       int32_t cnt4 = 0;
       for (int v = tid; v < n; v += kST) {
@@ -606,6 +783,158 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
       nvalid -= block_sum(cnt4, ctl);
     }
   }
+}
+
+// Components of an edge list in lab.  Every vertex first hooks under its
+// smallest neighbour, one minimum per edge and no walk; most edges then lie
+// inside one tree, while joining edge by edge from the start builds deep
+// trees that every later edge walks (52,000 edges: a call of 103 -> 86 us).
+// In CSR order the minima of a list meet in one word, and the plain joins are
+// faster (92 against 128 us).  Returns false for an id outside [0, n).
+__device__ __forceinline__ bool listed_wcc(const SmallDesc& D, int n, int32_t* lab, int32_t* ctl) {
+  for (int v = threadIdx.x; v < n; v += kST) lab[v] = v;
+  __syncthreads();
+  for_each_listed(D, [&](int32_t a, int32_t b) {
+    if ((unsigned)a >= (unsigned)n || (unsigned)b >= (unsigned)n) ctl[cBad] = 1;
+    else atomicMin(&lab[max(a, b)], min(a, b));
+  });
+  __syncthreads();
+  if (ctl[cBad]) return false;
+  for (int v = threadIdx.x; v < n; v += kST) lab[v] = uf_find(lab, v);
+  __syncthreads();
+  for_each_listed(D, [&](int32_t a, int32_t b) {
+    if ((unsigned)a >= (unsigned)n || (unsigned)b >= (unsigned)n) return;  // (changed since)
+    if (*(volatile int32_t*)(lab + a) != *(volatile int32_t*)(lab + b)) uf_unite(lab, a, b);
+  });
+  __syncthreads();
+  return true;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc* many,
+                                                  int32_t max_steps, int32_t colour_rounds,
+                                                  int* err) {
+  const SmallDesc D = many ? many[blockIdx.x] : one;
+  const int n = D.n;
+  if (n <= 0) return;
+  const int tid = threadIdx.x;
+  const SmallMem s = small_mem(n);
+  int32_t* const ctl = s.ctl;
+  int32_t* const ooff = s.ooff;
+  int32_t* const ioff = s.ioff;
+  int32_t* const lab = s.lab;
+  int32_t* const cnt_o = s.cnt_o;
+  int32_t* const cnt_i = s.cnt_i;
+  const int32_t cap = (int32_t)min((long long)max_steps, 4ll * n + 64);
+  if (tid == 0) {
+    ctl[cBad] = 0;
+    ctl[cStop] = 0;
+  }
+
+  // ---- WCC from an edge list: union-find over the edges, no CSR ----------
+  if (KIND == 1 && D.out_off == nullptr) {
+    __syncthreads();
+    if (!listed_wcc(D, n, lab, ctl)) {
+      if (tid == 0) atomicCAS(err, 0, (int)kErrInvalid);
+      return;
+    }
+    for (int v = tid; v < n; v += kST) D.labels[v] = uf_find(lab, v);
+    return;
+  }
+
+  // ---- the CSR ------------------------------------------------------------
+  SmallCsr g;
+  if (D.out_off != nullptr) {
+    const long long ob = D.out_off[0];
+    const long long ib = D.in_off ? D.in_off[0] : ob;
+    for (int v = tid; v <= n; v += kST) {
+      ooff[v] = (int32_t)(D.out_off[v] - ob);
+      ioff[v] = D.in_off ? (int32_t)(D.in_off[v] - ib) : ooff[v];
+    }
+    g.oadj = D.out_adj + ob;
+    g.iadj = D.in_off ? D.in_adj + ib : g.oadj;
+    g.base = D.id_base;
+  } else {
+    for (int v = tid; v < n; v += kST) {
+      cnt_o[v] = 0;
+      cnt_i[v] = 0;
+    }
+    __syncthreads();
+    for_each_listed(D, [&](int32_t a, int32_t b) {
+      if ((unsigned)a >= (unsigned)n || (unsigned)b >= (unsigned)n) {
+        ctl[cBad] = 1;
+      } else {
+        atomicAdd(&cnt_o[a], 1);
+        atomicAdd(&cnt_i[b], 1);
+      }
+    });
+    __syncthreads();
+    if (ctl[cBad]) {
+      if (tid == 0) atomicCAS(err, 0, (int)kErrInvalid);
+      return;
+    }
+    for (int v = tid; v < n; v += kST) {
+      ooff[v] = cnt_o[v];
+      ioff[v] = cnt_i[v];
+    }
+    if (tid == 0) {
+      ooff[n] = 0;
+      ioff[n] = 0;
+    }
+    block_scan(ooff, n + 1, ctl);
+    block_scan(ioff, n + 1, ctl);
+    for (int v = tid; v < n; v += kST) {
+      cnt_o[v] = ooff[v];
+      cnt_i[v] = ioff[v];
+    }
+    __syncthreads();
+    int32_t* so = D.adj_scratch;
+    int32_t* si = D.adj_scratch + D.m;
+    // (a list in host memory may be read twice with other values in between,
+    // by a caller that writes it under the call: no access leaves its array)
+    for_each_listed(D, [&](int32_t a, int32_t b) {
+      if ((unsigned)a >= (unsigned)n || (unsigned)b >= (unsigned)n) return;
+      const int32_t po = atomicAdd(&cnt_o[a], 1), pi = atomicAdd(&cnt_i[b], 1);
+      if (po < D.m) so[po] = b;
+      if (pi < D.m) si[pi] = a;
+    });
+    __syncthreads();
+    g.oadj = so;
+    g.iadj = si;
+    g.base = 0;
+  }
+  g.ooff = ooff;
+  g.ioff = ioff;
+
+  // ---- WCC on a CSR: union-find over the out-lists ------------------------
+  if (KIND == 1) {
+    for (int v = tid; v < n; v += kST) lab[v] = v;
+    __syncthreads();
+    for_each_edge(n, ooff, g.oadj, g.base, [&](int32_t u, int32_t w) { uf_unite(lab, u, w); });
+    __syncthreads();
+    for (int v = tid; v < n; v += kST) D.labels[v] = uf_find(lab, v);
+    return;
+  }
+
+  // ---- SCC ----------------------------------------------------------------
+  int32_t nvalid = -1;
+  int32_t hub = -1;
+  if (colour_rounds == kSigAfterSmall) {
+    // the vertex of largest out x in degree, among those with kHubDeg on
+    // both sides
+    long long key = -1;
+    int32_t id = 0x7fffffff;
+    __syncthreads();  // the offsets
+    for (int v = tid; v < n; v += kST) {
+      const int32_t od = ooff[v + 1] - ooff[v], idg = ioff[v + 1] - ioff[v];
+      const long long k = (long long)od * (long long)idg;
+      if (min(od, idg) >= kHubDeg && k > key) { key = k; id = v; }
+    }
+    if (__syncthreads_or(key >= 0)) hub = block_argmax(key, id, ctl);
+  }
+  if (hub >= 0)
+    nvalid = hub_scc(n, hub, g.oadj, g.iadj, g.base, cap);
+  if (nvalid != 0) queue_scc(n, g.oadj, g.iadj, g.base, cap, colour_rounds, nvalid);
   __syncthreads();
   if (ctl[cStop]) {
     if (tid == 0) atomicCAS(err, 0, (int)kErrIterLimit);
@@ -622,10 +951,10 @@ cudaError_t launch_k(const SmallDesc& one, const SmallDesc* many, int count, int
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const size_t smem = small_smem_bytes(max_n);
+  const size_t smem = small_smem_bytes(KIND, max_n);
   if (dev < 0 || dev >= 64 || !attr_set[dev][KIND]) {
     e = cudaFuncSetAttribute(k_small<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)small_smem_bytes(kSmallMaxN));
+                             (int)small_smem_bytes(KIND, kSmallMaxN));
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) attr_set[dev][KIND] = true;
   }
@@ -635,9 +964,12 @@ cudaError_t launch_k(const SmallDesc& one, const SmallDesc* many, int count, int
 
 }  // namespace
 
-size_t small_smem_bytes(int32_t max_n) {
+size_t small_smem_bytes(int kind, int32_t max_n) {
   const size_t n = (size_t)(max_n > 0 ? max_n : 1);
-  return (size_t)kCtlInts * 4 + (9 * n + 3) * 4;
+  const size_t all = (size_t)kCtlInts * 4 + (9 * n + 3) * 4;
+  // (offsets, labels and flags stay beside hub_scc's memory)
+  const size_t hub = (size_t)kCtlInts * 4 + (4 * n + 2 + 4) * 4 + kHubSmem;
+  return kind == 1 || all > hub ? all : hub;
 }
 
 cudaError_t launch_small(int kind, const SmallDesc& one, const SmallDesc* many, int count,
@@ -646,7 +978,7 @@ cudaError_t launch_small(int kind, const SmallDesc& one, const SmallDesc* many, 
   if (count <= 0) return cudaSuccess;
   if (max_n > kSmallMaxN) return cudaErrorInvalidValue;
   // colour rounds before the signature rounds: all (0), none (1), four (2)
-  const int32_t cr = colour_mode == 0 ? 0x7fffffff : (colour_mode == 1 ? 0 : 4);
+  const int32_t cr = colour_mode == 0 ? 0x7fffffff : (colour_mode == 1 ? 0 : kSigAfterSmall);
   return kind == 0 ? launch_k<0>(one, many, count, max_n, max_steps, cr, err, s)
                    : launch_k<1>(one, many, count, max_n, max_steps, cr, err, s);
 }
