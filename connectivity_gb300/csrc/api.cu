@@ -288,7 +288,6 @@ gb_status finish_run(gb_ctx* c, const gb_graph* g, gb_stats* st) {
     st->err_where = h.err_where;
   }
   *c->h_sticky = 0;
-  cudaMemsetAsync(c->d_sticky, 0, 2 * sizeof(int), c->stream);
   if (h.err != 0) {
     char buf[128];
     std::snprintf(buf, sizeof(buf), "device error %d at site %d", h.err, h.err_where);
@@ -325,13 +324,9 @@ gb_status run_small(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t* lab
   }
   gb_status s = ensure_ws(c, g->n);
   if (s != GB_OK) return s;
-  int32_t* dl = dev_labels ? labels : c->w.label;
   cudaStream_t sm = c->stream;
-  CK(cudaMemsetAsync(&c->d_ctl->err, 0, 2 * sizeof(int), sm), "memset");
-  cudaEvent_t* ev = c->ev[c->runs % gb_ctx::kRing];
-  CK(cudaMemsetAsync(c->d_tphase + 4 * (c->runs % gb_ctx::kRing), 0,
-                     4 * sizeof(unsigned long long), sm),
-     "memset");
+  const int slot = (int)(c->runs % gb_ctx::kRing);
+  cudaEvent_t* ev = c->ev[slot];
   c->runs++;
   cudaEventRecord(ev[0], sm);
   gb::SmallDesc d{};
@@ -341,20 +336,18 @@ gb_status run_small(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t* lab
   d.out_adj = g->out_adj;
   d.in_off = g->symmetric ? nullptr : g->in_off;
   d.in_adj = g->symmetric ? nullptr : g->in_adj;
-  d.labels = dl;
+  d.labels = dev_labels ? labels : c->h_small;
+  const gb::SmallStatus status{&c->d_ctl->err, c->d_sticky, wait, &c->h_ctl->err,
+                               c->d_tphase + 4 * slot};
   const int32_t max_steps = o && o->max_steps > 0 ? o->max_steps : (1 << 30);
-  CK(gb::launch_small(kind == gb::kSCC ? 0 : 1, d, nullptr, 1, g->n, max_steps, &c->d_ctl->err,
-                      sm, o ? o->colour_mode : 2),
+  CK(gb::launch_small(kind == gb::kSCC ? 0 : 1, d, nullptr, 1, g->n, max_steps, status, sm,
+                      o ? o->colour_mode : 2),
      "kernel launch");
   cudaEventRecord(ev[1], sm);
   cudaEventRecord(ev[4], sm);
-  CK(gb::launch_latch(c->d_ctl, c->d_sticky, sm), "kernel launch");
-  if (!dev_labels)
-    CK(cudaMemcpyAsync(labels, dl, (size_t)g->n * 4, cudaMemcpyDeviceToHost, sm), "labels copy");
-  CK(cudaMemcpyAsync(&c->h_ctl->err, &c->d_ctl->err, 2 * sizeof(int), cudaMemcpyDeviceToHost, sm),
-     "status copy");
   if (!wait) return GB_OK;
   CK(cudaStreamSynchronize(sm), "run");
+  if (!dev_labels && c->h_ctl->err == 0) std::memcpy(labels, c->h_small, (size_t)g->n * 4);
   if (st) {
     std::memset(st, 0, sizeof(*st));
     float tot = 0.f;
@@ -364,7 +357,6 @@ gb_status run_small(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t* lab
     st->err_where = c->h_ctl->err_where;
   }
   *c->h_sticky = 0;
-  cudaMemsetAsync(c->d_sticky, 0, 2 * sizeof(int), sm);
   const int err = c->h_ctl->err;
   if (err != 0) {
     gb_set_error("run: %s", err == gb::kErrIterLimit ? "a loop of the one-block path hit its step cap"
@@ -408,12 +400,12 @@ gb_status run_union_cc(gb_ctx* c, const gb_graph* g, int32_t* labels, gb_stats* 
   if (s != GB_OK) return s;
   int32_t* dl = dev_labels ? labels : c->w.label;
   cudaStream_t sm = c->stream;
-  CK(cudaMemsetAsync(&c->d_ctl->err, 0, 2 * sizeof(int), sm), "memset");
-  cudaEvent_t* ev = c->ev[c->runs % gb_ctx::kRing];
-  CK(cudaMemsetAsync(c->d_tphase + 4 * (c->runs % gb_ctx::kRing), 0,
-                     4 * sizeof(unsigned long long), sm),
-     "memset");
-  if (!sampled) CK(cudaMemsetAsync(&c->d_ctl->uf_cross, 0, 8, sm), "memset");
+  const int slot = (int)(c->runs % gb_ctx::kRing);
+  cudaEvent_t* ev = c->ev[slot];
+  gb::Fills fills;
+  fills.add(c->d_ctl, sizeof(gb::Ctl));
+  fills.add(c->d_tphase + 4 * slot, 4 * sizeof(unsigned long long));
+  CK(gb::launch_fills(fills, sm), "kernel launch");
   c->runs++;
   cudaEventRecord(ev[0], sm);
   // (a checked device graph: the id flag, err_where, stays clear)
@@ -427,11 +419,9 @@ gb_status run_union_cc(gb_ctx* c, const gb_graph* g, int32_t* labels, gb_stats* 
        "kernel launch");
   cudaEventRecord(ev[1], sm);
   cudaEventRecord(ev[4], sm);
-  CK(gb::launch_latch(c->d_ctl, c->d_sticky, sm), "kernel launch");
+  CK(gb::launch_latch(c->d_ctl, c->d_sticky, sm, c->h_ctl, wait), "kernel launch");
   if (!dev_labels)
     CK(cudaMemcpyAsync(labels, dl, (size_t)g->n * 4, cudaMemcpyDeviceToHost, sm), "labels copy");
-  CK(cudaMemcpyAsync(&c->h_ctl->err, &c->d_ctl->err, 2 * sizeof(int), cudaMemcpyDeviceToHost, sm),
-     "status copy");
   if (!wait) return GB_OK;
   CK(cudaStreamSynchronize(sm), "run");
   if (st) {
@@ -442,7 +432,6 @@ gb_status run_union_cc(gb_ctx* c, const gb_graph* g, int32_t* labels, gb_stats* 
     st->err_where = c->h_ctl->err_where;
   }
   *c->h_sticky = 0;
-  cudaMemsetAsync(c->d_sticky, 0, 2 * sizeof(int), sm);
   const int err = c->h_ctl->err;
   if (err != 0) {
     gb_set_error("run: %s", "a union-find link ran out of retries");
@@ -510,27 +499,26 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
   }
   gv.batch = gb::BatchView{};
   cudaStream_t sm = c->stream;
+  const int slot = (int)(c->runs % gb_ctx::kRing);
+  cudaEvent_t* ev = c->ev[slot];
+  w.tphase = c->d_tphase + 4 * slot;
+  gb::Fills fills;
+  fills.add(c->d_ctl, sizeof(gb::Ctl));
+  fills.add(w.tphase, 4 * sizeof(unsigned long long));
+  // (the reached and done bitmaps are adjacent in the workspace)
+  fills.add(w.fvis, (size_t)((char*)(w.done + w.nwords) - (char*)w.fvis));
   if (bv != nullptr) {
     gv.batch = *bv;
-    CK(cudaMemsetAsync(bv->pkey, 0, (size_t)bv->count * 8, sm), "memset");
-    CK(cudaMemsetAsync(bv->gmin, 0x7f, (size_t)bv->count * 4, sm), "memset");
+    fills.add(bv->pkey, (size_t)bv->count * 8);
+    fills.add(bv->gmin, (size_t)bv->count * 4, 0x7f7f7f7fu);
   }
-  // the reached and done bitmaps are adjacent in the workspace: one memset
-  // clears all three
-  CK(cudaMemsetAsync(c->d_ctl, 0, sizeof(gb::Ctl), sm), "memset");
-  CK(cudaMemsetAsync(w.fvis, 0,
-                     (size_t)((char*)(w.done + w.nwords) - (char*)w.fvis), sm),
-     "memset");
-  cudaEvent_t* ev = c->ev[c->runs % gb_ctx::kRing];
-  w.tphase = c->d_tphase + 4 * (c->runs % gb_ctx::kRing);
-  CK(cudaMemsetAsync(w.tphase, 0, 4 * sizeof(unsigned long long), sm), "memset");
+  CK(gb::launch_fills(fills, sm), "kernel launch");
   c->runs++;
   CK(gb::launch_run(gv, kind, p, w, grid, sm, ev), "kernel launch");
-  CK(gb::launch_latch(c->d_ctl, c->d_sticky, sm), "kernel launch");
+  CK(gb::launch_latch(c->d_ctl, c->d_sticky, sm, c->h_ctl, wait), "kernel launch");
   if (bv != nullptr) CK(gb::launch_localize(w.label, g->n, bv->gid, bv->vbase, sm), "localize");
   if (!dev_labels)
     CK(cudaMemcpyAsync(labels, w.label, (size_t)g->n * 4, cudaMemcpyDeviceToHost, sm), "labels copy");
-  CK(cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(gb::Ctl), cudaMemcpyDeviceToHost, sm), "status copy");
   if (!wait) return GB_OK;
   return finish_run(c, g, st);
 }
@@ -625,7 +613,8 @@ gb_status gb_ctx_create(int device, gb_ctx** out) {
     if ((r = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking)) != cudaSuccess) { s = cuda_fail(r, "stream"); break; }
     c->stream = c->own;
     if ((r = cudaMalloc(&c->d_ctl, sizeof(gb::Ctl))) != cudaSuccess) { s = cuda_fail(r, "ctl"); break; }
-    if ((r = cudaMallocHost(&c->h_ctl, sizeof(gb::Ctl))) != cudaSuccess) { s = cuda_fail(r, "ctl"); break; }
+    if ((r = cudaMallocHost(&c->h_ctl, sizeof(gb::Ctl) + gb::kSmallMaxN * 4)) != cudaSuccess) { s = cuda_fail(r, "ctl"); break; }
+    c->h_small = reinterpret_cast<int32_t*>(c->h_ctl + 1);
     if ((r = cudaMalloc(&c->d_sticky, 2 * sizeof(int))) != cudaSuccess) { s = cuda_fail(r, "sticky"); break; }
     const size_t pr = sizeof(unsigned long long) * 4 * gb_ctx::kRing;
     if ((r = cudaMalloc(&c->d_tphase, pr)) != cudaSuccess) { s = cuda_fail(r, "phase ring"); break; }
@@ -1255,7 +1244,7 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   // CSR built by the block (2m ints) and the labels (for host labels)
   const size_t edge_b = dev_edges ? 0 : (size_t)m * 8;
   const size_t scr_b = kind == gb::kSCC ? (size_t)m * 8 : 0;  // (the one-block SCC)
-  const size_t lab_b = dev_labels ? 0 : (size_t)n * 4;
+  const size_t lab_b = dev_labels || small ? 0 : (size_t)n * 4;  // (one block: h_small)
   char* buf = nullptr;
   if (edge_b + scr_b + lab_b > 0)
     CK(cudaMallocAsync((void**)&buf, edge_b + scr_b + lab_b, sm), "edge staging");
@@ -1274,24 +1263,30 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
     sd.dst = ds + m;
   }
   sd.adj_scratch = scr_b ? reinterpret_cast<int32_t*>(buf + edge_b) : nullptr;
-  sd.labels = dev_labels ? labels : reinterpret_cast<int32_t*>(buf + edge_b + scr_b);
+  sd.labels = dev_labels ? labels
+              : small    ? c->h_small
+                         : reinterpret_cast<int32_t*>(buf + edge_b + scr_b);
   const int32_t max_steps = o->max_steps > 0 ? o->max_steps : (1 << 30);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&c->d_ctl->err, 0, 2 * sizeof(int), sm);
-  if (e == cudaSuccess && uni)
-    e = gb::cc_union_edges(n, m, sd.src, sd.dst, sd.labels, &c->d_ctl->err, sm);
-  if (e == cudaSuccess && !uni)
-    e = gb::launch_small(kind == gb::kSCC ? 0 : 1, sd, nullptr, 1, n, max_steps, &c->d_ctl->err,
-                         sm, o->colour_mode);
-  if (e == cudaSuccess && !dev_labels)
-    e = cudaMemcpyAsync(labels, sd.labels, (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&c->h_ctl->err, &c->d_ctl->err, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                        sm);
+  if (small) {
+    if (e == cudaSuccess)
+      e = gb::launch_small(kind == gb::kSCC ? 0 : 1, sd, nullptr, 1, n, max_steps,
+                           {&c->d_ctl->err, nullptr, false, &c->h_ctl->err}, sm, o->colour_mode);
+  } else {
+    if (e == cudaSuccess) e = cudaMemsetAsync(&c->d_ctl->err, 0, 2 * sizeof(int), sm);
+    if (e == cudaSuccess)
+      e = gb::cc_union_edges(n, m, sd.src, sd.dst, sd.labels, &c->d_ctl->err, sm);
+    if (e == cudaSuccess && !dev_labels)
+      e = cudaMemcpyAsync(labels, sd.labels, (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(&c->h_ctl->err, &c->d_ctl->err, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+                          sm);
+  }
   if (buf) cudaFreeAsync(buf, sm);
   const cudaError_t e2 = cudaStreamSynchronize(sm);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return cuda_fail(e, "run from edges");
   const int err = c->h_ctl->err;
+  if (small && !dev_labels && err == 0) std::memcpy(labels, c->h_small, (size_t)n * 4);
   if (err != 0) {
     gb_set_error("run from edges: %s", err == gb::kErrInvalid ? "vertex id outside [0, n)"
                                                               : "a loop hit its step cap");

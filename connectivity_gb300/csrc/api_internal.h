@@ -22,7 +22,8 @@ struct gb_ctx {
   unsigned long long* con_ws = nullptr;  // contraction's edge pairs (2 x con_cap)
   int64_t con_cap = 0;
   gb::Ctl* d_ctl = nullptr;
-  gb::Ctl* h_ctl = nullptr;     // pinned
+  gb::Ctl* h_ctl = nullptr;     // pinned; behind it h_small
+  int32_t* h_small = nullptr;   // kSmallMaxN labels, written by the one-block kernel
   int* d_sticky = nullptr;      // first error of any run since the last sync
   int* h_sticky = nullptr;      // pinned; [2]: verdict of an edge list's id check
   cudaEvent_t checked = nullptr;  // after that check

@@ -555,11 +555,29 @@ __global__ void k_pivot_min(int32_t n, const int64_t* out_off, const int64_t* in
   }
 }
 
-__global__ void k_latch(const Ctl* c, int* sticky) {
-  if (c->err != 0 && sticky[0] == 0) {
-    sticky[0] = c->err;
-    sticky[1] = c->err_where;
+// The end of a run: the error latch, and the control block into pinned host
+// memory (a copy and, after the wait, a memset less per run).
+__global__ void k_latch(const Ctl* c, int* sticky, uint32_t* host, bool clear) {
+  static_assert(sizeof(Ctl) % 4 == 0, "copied by words");
+  if (threadIdx.x == 0) {
+    if (clear) {
+      sticky[0] = sticky[1] = 0;
+    } else if (c->err != 0 && sticky[0] == 0) {
+      sticky[0] = c->err;
+      sticky[1] = c->err_where;
+    }
   }
+  if (host != nullptr)
+    for (int i = threadIdx.x; i < (int)(sizeof(Ctl) / 4); i += blockDim.x)
+      host[i] = reinterpret_cast<const uint32_t*>(c)[i];
+}
+
+// (three to five memsets of a few microseconds each in one launch)
+__global__ void k_fills(Fills f) {
+  const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int k = 0; k < f.count; ++k)
+    for (size_t i = t0; i < f.f[k].bytes / 4; i += (size_t)gridDim.x * blockDim.x)
+      static_cast<uint32_t*>(f.f[k].p)[i] = f.f[k].v;
 }
 
 // Degree key of the hint rule: the total degree itself below 32, above it
@@ -1114,8 +1132,16 @@ cudaError_t max_degrees(int32_t n, const int64_t* off0, const int64_t* off1, cud
   return cudaStreamSynchronize(s);
 }
 
-cudaError_t launch_latch(Ctl* ctl, int* sticky, cudaStream_t s) {
-  k_latch<<<1, 1, 0, s>>>(ctl, sticky);
+cudaError_t launch_latch(Ctl* ctl, int* sticky, cudaStream_t s, Ctl* host, bool clear) {
+  k_latch<<<1, host ? 512 : 32, 0, s>>>(ctl, sticky, reinterpret_cast<uint32_t*>(host), clear);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fills(const Fills& f, cudaStream_t s) {
+  size_t words = 0;
+  for (int k = 0; k < f.count; ++k) words = f.f[k].bytes / 4 > words ? f.f[k].bytes / 4 : words;
+  const size_t blocks = (words + 1023) / 1024;  // four words a thread, up to 152 x 4 blocks
+  k_fills<<<(unsigned)(blocks < 1 ? 1 : (blocks > 608 ? 608 : blocks)), 256, 0, s>>>(f);
   return cudaGetLastError();
 }
 

@@ -260,7 +260,24 @@ cudaError_t pivot_device(int32_t n, const int64_t* out_off, const int64_t* in_of
                          cudaStream_t s, int32_t* pivot);
 // Copies the first device error of a run into sticky[0..1] (code, site)
 // unless an earlier one is already there.
-cudaError_t launch_latch(Ctl* ctl, int* sticky, cudaStream_t s);
+// host non-null: the control block is copied there (pinned memory); clear: the
+// latch is cleared instead (a run that the host waits for reads its own error).
+cudaError_t launch_latch(Ctl* ctl, int* sticky, cudaStream_t s, Ctl* host = nullptr,
+                         bool clear = false);
+// Regions of 32-bit words set to one value each, in one launch (what a run
+// needs cleared before it starts).
+struct Fill {
+  void* p;
+  size_t bytes;
+  uint32_t v;
+};
+struct Fills {
+  static constexpr int kMax = 5;
+  Fill f[kMax];
+  int count = 0;
+  void add(void* p, size_t bytes, uint32_t v = 0) { f[count++] = {p, bytes, v}; }
+};
+cudaError_t launch_fills(const Fills& f, cudaStream_t s);
 
 // Small graphs, one thread block per graph (small.cu).  A graph of at most
 // kSmallMaxN vertices keeps its per-vertex state in shared memory.
@@ -288,14 +305,23 @@ struct SmallDesc {
 // Dynamic shared memory of a block for graphs of at most max_n vertices
 // (kind as for launch_small).
 size_t small_smem_bytes(int kind, int32_t max_n);
+// Where a run of one graph leaves its status; the kernel writes all of it, so
+// that no memset, latch or copy goes with the launch.
+struct SmallStatus {
+  int* err;                     // err and err_where
+  int* sticky = nullptr;        // the latch of asynchronous errors: set by an
+  bool clear = false;           // error, or cleared (a run that the host waits for)
+  int* host = nullptr;          // copy of err and err_where in pinned memory
+  unsigned long long* tphase = nullptr;  // four phase times, cleared
+};
 // kind 0 = SCC, 1 = WCC.  One block per graph: `count` descriptors from
 // `many` (device memory), or `one` when many is null (count 1).  A failure
 // (an id outside [0, n) in edge form: kErrInvalid; a loop past max_steps:
-// kErrIterLimit) is written to *err with atomicCAS from 0.  colour_mode as
-// in gb_opts: 0 colour rounds to the end, 1 signature rounds, 2 four colour
-// rounds and signature rounds for the rest.
+// kErrIterLimit) goes to st; with `many`, to *st.err alone, with atomicCAS
+// from 0.  colour_mode as in gb_opts: 0 colour rounds to the end, 1 signature
+// rounds, 2 four colour rounds and signature rounds for the rest.
 cudaError_t launch_small(int kind, const SmallDesc& one, const SmallDesc* many, int count,
-                         int32_t max_n, int32_t max_steps, int* err, cudaStream_t s,
+                         int32_t max_n, int32_t max_steps, const SmallStatus& st, cudaStream_t s,
                          int32_t colour_mode = 2);
 cudaError_t widen_offsets(const uint32_t* in, int64_t* out, int64_t count, cudaStream_t s);
 // Reference-layout CSR (32-bit offsets) from device-readable host memory into

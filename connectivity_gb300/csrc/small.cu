@@ -810,10 +810,32 @@ __device__ __forceinline__ bool listed_wcc(const SmallDesc& D, int n, int32_t* l
   return true;
 }
 
+// The run's status (one thread calls, once).  The kernel's own stores stand for
+// two memsets, a latch kernel and two copies around it, which were 10 of the
+// 50 us of a call.
+__device__ __forceinline__ void small_status(const SmallStatus& st, bool many, int code) {
+  if (many) {
+    if (code) atomicCAS(st.err, 0, code);
+    return;
+  }
+  st.err[0] = code;
+  st.err[1] = 0;
+  if (st.sticky) {
+    if (st.clear) st.sticky[0] = st.sticky[1] = 0;
+    else if (code && st.sticky[0] == 0) st.sticky[0] = code;
+  }
+  if (st.host) {
+    st.host[0] = code;
+    st.host[1] = 0;
+  }
+  if (st.tphase)
+    for (int i = 0; i < 4; ++i) st.tphase[i] = 0;
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc* many,
                                                   int32_t max_steps, int32_t colour_rounds,
-                                                  int* err) {
+                                                  SmallStatus st) {
   const SmallDesc D = many ? many[blockIdx.x] : one;
   const int n = D.n;
   if (n <= 0) return;
@@ -834,10 +856,9 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
   // ---- WCC from an edge list: union-find over the edges, no CSR ----------
   if (KIND == 1 && D.out_off == nullptr) {
     __syncthreads();
-    if (!listed_wcc(D, n, lab, ctl)) {
-      if (tid == 0) atomicCAS(err, 0, (int)kErrInvalid);
-      return;
-    }
+    const bool fine = listed_wcc(D, n, lab, ctl);
+    if (tid == 0) small_status(st, many != nullptr, fine ? 0 : (int)kErrInvalid);
+    if (!fine) return;
     for (int v = tid; v < n; v += kST) D.labels[v] = uf_find(lab, v);
     return;
   }
@@ -870,7 +891,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
     });
     __syncthreads();
     if (ctl[cBad]) {
-      if (tid == 0) atomicCAS(err, 0, (int)kErrInvalid);
+      if (tid == 0) small_status(st, many != nullptr, (int)kErrInvalid);
       return;
     }
     for (int v = tid; v < n; v += kST) {
@@ -913,6 +934,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
     for_each_edge(n, ooff, g.oadj, g.base, [&](int32_t u, int32_t w) { uf_unite(lab, u, w); });
     __syncthreads();
     for (int v = tid; v < n; v += kST) D.labels[v] = uf_find(lab, v);
+    if (tid == 0) small_status(st, many != nullptr, 0);
     return;
   }
 
@@ -936,16 +958,16 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
     nvalid = hub_scc(n, hub, g.oadj, g.iadj, g.base, cap);
   if (nvalid != 0) queue_scc(n, g.oadj, g.iadj, g.base, cap, colour_rounds, nvalid);
   __syncthreads();
-  if (ctl[cStop]) {
-    if (tid == 0) atomicCAS(err, 0, (int)kErrIterLimit);
-    return;
-  }
+  const bool stopped = ctl[cStop] != 0;
+  if (tid == 0) small_status(st, many != nullptr, stopped ? (int)kErrIterLimit : 0);
+  if (stopped) return;
   for (int v = tid; v < n; v += kST) D.labels[v] = lab[v];
 }
 
 template <int KIND>
 cudaError_t launch_k(const SmallDesc& one, const SmallDesc* many, int count, int32_t max_n,
-                     int32_t max_steps, int32_t colour_rounds, int* err, cudaStream_t s) {
+                     int32_t max_steps, int32_t colour_rounds, const SmallStatus& st,
+                     cudaStream_t s) {
   // the shared-memory attribute, once per device
   static bool attr_set[64][2] = {};
   int dev = 0;
@@ -958,7 +980,7 @@ cudaError_t launch_k(const SmallDesc& one, const SmallDesc* many, int count, int
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) attr_set[dev][KIND] = true;
   }
-  k_small<KIND><<<count, kST, smem, s>>>(one, many, max_steps, colour_rounds, err);
+  k_small<KIND><<<count, kST, smem, s>>>(one, many, max_steps, colour_rounds, st);
   return cudaGetLastError();
 }
 
@@ -973,14 +995,14 @@ size_t small_smem_bytes(int kind, int32_t max_n) {
 }
 
 cudaError_t launch_small(int kind, const SmallDesc& one, const SmallDesc* many, int count,
-                         int32_t max_n, int32_t max_steps, int* err, cudaStream_t s,
+                         int32_t max_n, int32_t max_steps, const SmallStatus& st, cudaStream_t s,
                          int32_t colour_mode) {
   if (count <= 0) return cudaSuccess;
   if (max_n > kSmallMaxN) return cudaErrorInvalidValue;
   // colour rounds before the signature rounds: all (0), none (1), four (2)
   const int32_t cr = colour_mode == 0 ? 0x7fffffff : (colour_mode == 1 ? 0 : kSigAfterSmall);
-  return kind == 0 ? launch_k<0>(one, many, count, max_n, max_steps, cr, err, s)
-                   : launch_k<1>(one, many, count, max_n, max_steps, cr, err, s);
+  return kind == 0 ? launch_k<0>(one, many, count, max_n, max_steps, cr, st, s)
+                   : launch_k<1>(one, many, count, max_n, max_steps, cr, st, s);
 }
 
 }  // namespace gb
