@@ -958,8 +958,8 @@ def headline(gb, ctx, stream, args, ws, rank, local, barrier, allmax):
         "autotuned": autotuned,
         "phases_ms": {k: round(float(v), 4) for k, v in
                       zip(("trim", "reach", "colour", "tail", "total"), pm)},
-        "gpu_launches": 2 * K,
-        "gpu_launches_note": "k_run (one cooperative launch) and the status latch per step",
+        "gpu_launches": 3 * K,
+        "gpu_launches_note": "k_fills, k_run (one cooperative launch) and k_latch per step",
         "clocks": ck,
     }
     if rank == 0 and ws == 1 and not args.no_cpu_baseline:
