@@ -32,7 +32,7 @@ CU_SOURCES = ["kernels.cu", "kernels_options.cu", "kernels_contract.cu",
               "csr_build.cu", "csr_part.cu", "api.cu", "batch.cu", "noalloc.cu", "serve.cu",
               "ingest.cu", "tune.cu", "small.cu", "afforest.cu", "unionfind.cu"]
 CPP_SOURCES = ["host_util.cpp"]
-HEADERS = ["gb_internal.cuh", "run_device.cuh", "run_kernel.cuh", "contract_device.cuh", "residual_device.cuh", "gen_common.h", "host_internal.h", "api_internal.h"]
+HEADERS = ["gb_internal.cuh", "append_slot.h", "run_device.cuh", "run_kernel.cuh", "contract_device.cuh", "residual_device.cuh", "gen_common.h", "host_internal.h", "api_internal.h"]
 
 
 def _nvcc() -> str:

@@ -129,16 +129,16 @@ struct ConStage {
   int n;
 };
 __device__ __forceinline__ void con_flush(ConStage& s, unsigned long long* arr, long long base,
-                                          long long dir, long long cap, int32_t* counter,
+                                          long long dir, long long cap, append_count* counter,
                                           int32_t* over) {
   __syncwarp();
   if (s.n > 0) {
-    int pos = 0;
-    if (lane_id() == 0) pos = atomicAdd(counter, s.n);
+    append_count pos = 0;
+    if (lane_id() == 0) pos = atomicAdd(counter, (append_count)s.n);
     pos = __shfl_sync(kFull, pos, 0);
     for (int i = lane_id(); i < s.n; i += 32) {
-      const long long at = (long long)pos + i;
-      if (at < cap) arr[base + dir * at] = s.buf[i];
+      const long long at = append_slot(pos, (unsigned)i, cap);
+      if (at >= 0) arr[base + dir * at] = s.buf[i];
       else *over = 1;
     }
   }
@@ -148,16 +148,17 @@ __device__ __forceinline__ void con_flush(ConStage& s, unsigned long long* arr, 
 template <bool kStaged>
 __device__ __forceinline__ void con_push(ConStage& s, bool flag, int32_t a, int32_t b,
                                          unsigned long long* arr, long long base, long long dir,
-                                         long long cap, int32_t* counter, int32_t* over) {
+                                         long long cap, append_count* counter, int32_t* over) {
   const unsigned mask = __ballot_sync(kFull, flag);
   if (mask == 0u) return;
   const int cnt = __popc(mask);
   if constexpr (!kStaged) {
-    int pos = 0;
-    if (lane_id() == 0) pos = atomicAdd(counter, cnt);
-    pos = __shfl_sync(kFull, pos, 0) + __popc(mask & lanemask_lt());
+    append_count pos = 0;
+    if (lane_id() == 0) pos = atomicAdd(counter, (append_count)cnt);
+    pos = __shfl_sync(kFull, pos, 0);
     if (flag) {
-      if (pos < cap) arr[base + dir * pos] = ((unsigned long long)(uint32_t)a << 32) | (uint32_t)b;
+      const long long at = append_slot(pos, (unsigned)__popc(mask & lanemask_lt()), cap);
+      if (at >= 0) arr[base + dir * at] = ((unsigned long long)(uint32_t)a << 32) | (uint32_t)b;
       else *over = 1;
     }
     return;
@@ -238,9 +239,9 @@ struct Contract {
   long long lcap;
   // per round: |A_t|, |E_t|, end of D and of the log after round t
   int32_t* cntA;
-  int32_t* cntE;
+  append_count* cntE;
   int32_t* cntD;
-  int32_t* cntL;
+  append_count* cntL;
   int32_t* over;    // an array ran out: the round is undone
 };
 
@@ -412,8 +413,8 @@ template <class W>
 __device__ __noinline__ bool con_undo(const Contract& k, const W& w, int t) {
   const long long tid = w.tid(), nth = w.threads();
   const uint32_t stH = con_state(t, kConHook);
-  const int32_t l0 = t > 0 ? W::ld(k.cntL + t) : 0;
-  const int32_t l1 = (int32_t)min((long long)W::ld(k.cntL + t + 1), k.lcap);
+  const long long l0 = t > 0 ? (long long)W::ld(k.cntL + t) : 0;
+  const long long l1 = min((long long)W::ld(k.cntL + t + 1), k.lcap);
   const int32_t d0 = t > 0 ? W::ld(k.cntD + t) : 0, d1 = W::ld(k.cntD + t + 1);
   for (long long i = l0 + tid; i < l1; i += nth) {
     const unsigned long long e = W::ld(k.elog + i);
@@ -463,7 +464,7 @@ struct ConLocal {
   int t;
   template <class W, class F>
   __device__ __forceinline__ void edges(const W& w, F f) const {
-    const int32_t ne = __ldcg(k->cntE + t);
+    const int32_t ne = (int32_t)__ldcg(k->cntE + t);  // (at most kConTailEdges)
     for (int32_t b = (int32_t)w.tid() & ~31; b < ne; b += (int32_t)w.threads()) {
       const int32_t i = b + (int32_t)lane_id();
       int32_t s = 0, d = 0;
@@ -483,7 +484,7 @@ struct ConLocal {
 // (out.x) of equal pairs; a vertex whose two agree is in that id's component.
 template <class W>
 __device__ __forceinline__ bool con_core(const Contract& k, const W& w, int t, volatile int* flag) {
-  const int32_t na = W::ld(k.cntA + t), ne = W::ld(k.cntE + t);
+  const int32_t na = W::ld(k.cntA + t), ne = (int32_t)W::ld(k.cntE + t);
   const int tid = (int)w.tid(), nth = (int)w.threads();
   for (int i = tid; i < na; i += nth) {
     const int32_t v = con_vertex<W>(k, t, i);
@@ -547,7 +548,8 @@ template <int32_t V, int32_t E, int32_t L, class Src>
 __device__ __noinline__ int con_solve(const Src& src, int32_t n, int32_t* smem,
                                       volatile int* left, int32_t** comp) {
   __shared__ int s_flag;
-  __shared__ int32_t s_cnt[4][kConRounds + 2];
+  __shared__ int32_t s_cnt[2][kConRounds + 2];
+  __shared__ append_count s_ecnt[2][kConRounds + 2];
   __shared__ int32_t s_over;
   const int tid = threadIdx.x, nth = blockDim.x;
   Contract l;
@@ -566,13 +568,16 @@ __device__ __noinline__ int con_solve(const Src& src, int32_t n, int32_t* smem,
   l.list0 = nullptr;
   l.n0 = n;
   l.cntA = s_cnt[0];
-  l.cntE = s_cnt[1];
-  l.cntD = s_cnt[2];
-  l.cntL = s_cnt[3];
+  l.cntD = s_cnt[1];
+  l.cntE = s_ecnt[0];
+  l.cntL = s_ecnt[1];
   l.over = &s_over;
   *comp = l.tc;
   if (tid == 0) s_over = 0;
-  for (int i = tid; i < 4 * (kConRounds + 2); i += nth) (&s_cnt[0][0])[i] = 0;
+  for (int i = tid; i < 2 * (kConRounds + 2); i += nth) {
+    (&s_cnt[0][0])[i] = 0;
+    (&s_ecnt[0][0])[i] = 0;
+  }
   for (int i = tid; i < n; i += nth) {
     l.in[i] = make_int2(kConInf, -1);
     l.out[i] = make_int2(kConInf, -1);
@@ -738,9 +743,9 @@ __device__ __noinline__ void contract_phase(const Args& A, Smem& sm) {
   k.elog = w.con_edges + w.con_cap;
   k.lcap = w.con_cap;
   k.cntA = c->con_cnt[0];
-  k.cntE = c->con_cnt[1];
-  k.cntD = c->con_cnt[2];
-  k.cntL = c->con_cnt[3];
+  k.cntD = c->con_cnt[1];
+  k.cntE = c->con_ecnt[0];
+  k.cntL = c->con_ecnt[1];
   k.over = &c->con_over;
   Steps st = steps_open(c);
   trace_rec(c, nl, 20);

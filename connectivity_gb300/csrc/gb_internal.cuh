@@ -4,6 +4,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "append_slot.h"
 #include "gen_common.h"
 
 namespace gb {
@@ -115,13 +116,15 @@ struct Ctl {
   // Diagnostic: device time at which each block finished the thread tier of
   // the first pull step of the run.
   unsigned long long blk_t[256];
-  // contraction rounds (contract_device.cuh): per round the vertices and
-  // edges alive, the vertices merged and the edges logged so far
-  int32_t con_cnt[4][kConRounds + 2];
+  // contraction rounds (contract_device.cuh): per round the vertices alive
+  // and merged so far, and the edges alive and logged so far
+  int32_t con_cnt[2][kConRounds + 2];
+  append_count con_ecnt[2][kConRounds + 2];
   int32_t con_over;   // an array ran out
   int32_t con_big;    // a vertex has too many edges
   int32_t con_open;   // vertices left without a component
-  int32_t res_cnt[2][2];  // residual: vertices and edges, before and after its trim
+  int32_t res_cnt[2];     // residual: vertices, before and after its trim
+  append_count res_ecnt[2];  // and edges
   int32_t res_over;       // an edge list ran out
   int32_t res_ready;      // its per-vertex state was set by the compaction
   int32_t con_may;    // sampled vertices that the first round may merge

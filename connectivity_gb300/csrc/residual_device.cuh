@@ -24,7 +24,7 @@ struct ResidVisit {
   int32_t* flag;  // bit 0: has an out-edge, bit 1: has an in-edge
   unsigned long long* list;
   long long cap;
-  int32_t* count;
+  append_count* count;
   int32_t* over;
   __device__ __forceinline__ int32_t source(int32_t v) const { return v; }
   __device__ __forceinline__ void edges(const int32_t (&sv)[kEU], const int32_t (&w)[kEU],
@@ -67,8 +67,8 @@ __device__ __noinline__ bool residual_phase(const Args& A, Smem& sm) {
   k.tc = w.candA;
   k.arena = reinterpret_cast<unsigned long long*>(w.listB);
   k.acap = w.n / 2;
-  k.cntA = c->res_cnt[0];
-  k.cntE = c->res_cnt[1];
+  k.cntA = c->res_cnt;
+  k.cntE = c->res_ecnt;
   int32_t* const over = &c->res_over;
   trace_rec(c, nl, 28);
   if (!__ldcg(&c->res_ready)) {  // (no search ran, so no compaction did)
@@ -97,7 +97,7 @@ __device__ __noinline__ bool residual_phase(const Args& A, Smem& sm) {
     }
   }
   const bool lost = __ldcg(over) != 0;
-  const int32_t ne0 = __ldcg(k.cntE);
+  const long long ne0 = (long long)__ldcg(k.cntE);
   for (long long base = tid & ~31ll; base < nl; base += nth) {
     const long long i = base + lane_id();
     int32_t v = 0;
@@ -123,7 +123,8 @@ __device__ __noinline__ bool residual_phase(const Args& A, Smem& sm) {
     }
   }
   if (!step_sync(c, st, 504)) return false;
-  const int32_t na = __ldcg(k.cntA + 1), ne = __ldcg(k.cntE + 1);
+  const int32_t na = __ldcg(k.cntA + 1);
+  const append_count ne = __ldcg(k.cntE + 1);
   const bool tail = na <= kConTailVerts && ne <= kConTailEdges && __ldcg(over) == 0;
   bool done = na == 0;
   trace_rec(c, na, 29);
