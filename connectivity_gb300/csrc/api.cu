@@ -484,7 +484,7 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
       g->m <= 5 * (int64_t)g->n && p.fwbw_rounds == 1 && p.tune.expand_mode == 0) {
     if ((s = ensure_con(c, g->m)) != GB_OK) return s;
     w.con_edges = c->con_ws;
-    w.con_cap = c->con_cap;
+    w.con_cap = g->m;  // (not what an earlier graph left: the result's route is this graph's)
   }
   int grid = c->grid;
   if (o && o->grid_blocks > 0 && o->grid_blocks < grid) grid = o->grid_blocks;

@@ -665,12 +665,13 @@ __device__ __noinline__ bool contract_run(const Contract& k, const Src& src, Ctl
     ++t;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *rounds = t;
+  // (an array may run out in the very round that leaves no vertex alive)
   const bool undone = __ldcg(k.over) != 0;
-  if (small) {
+  if (undone || !pays) {
+    con_open(k, g, t, undone);
+  } else if (small) {
     trace_rec(c, __ldcg(k.cntA + t), 23);
     if (blockIdx.x == 0) con_tail(k, c, t, max_steps - (st.s - st.s0), smem, rounds);
-  } else if (!pays) {
-    con_open(k, g, t, undone);
   }
   trace_rec(c, t, 24);
   if (!g.sync(430)) return false;
