@@ -1233,17 +1233,21 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   const bool dev_labels = is_device_ptr(labels);
   // a short list in host memory that the device reads is used in place: two
   // copies cost more than the block's reads over the host link
+  bool in_place = false;
   if (small && !dev_edges && m <= gb::kSmallAutoEdges) {
     const void *vs = host_view(src), *vd = host_view(dst);
     if (vs && vd) {
       src = (const int32_t*)vs;
       dst = (const int32_t*)vd;
       dev_edges = true;
+      in_place = true;
     }
   }
-  // one stream-ordered allocation: the edges (from host memory), the SCC
-  // CSR built by the block (2m ints) and the labels (for host labels)
-  const size_t edge_b = dev_edges ? 0 : (size_t)m * 8;
+  // one stream-ordered allocation: the edges (from host memory, or as the
+  // block reads them there), the SCC CSR built by the block (2m ints) and the
+  // labels (for host labels)
+  const bool keep = in_place && kind == gb::kSCC;
+  const size_t edge_b = dev_edges && !keep ? 0 : (size_t)m * 8;
   const size_t scr_b = kind == gb::kSCC ? (size_t)m * 8 : 0;  // (the one-block SCC)
   const size_t lab_b = dev_labels || small ? 0 : (size_t)n * 4;  // (one block: h_small)
   char* buf = nullptr;
@@ -1263,6 +1267,7 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
     sd.src = ds;
     sd.dst = ds + m;
   }
+  if (keep) sd.kept = reinterpret_cast<int32_t*>(buf);
   sd.adj_scratch = scr_b ? reinterpret_cast<int32_t*>(buf + edge_b) : nullptr;
   sd.labels = dev_labels ? labels
               : small    ? c->h_small

@@ -6,9 +6,9 @@
 #include <cstdint>
 
 #ifdef __CUDACC__
-#define GB_HD __host__ __device__ __forceinline__
+#define GB_HOST_DEVICE __host__ __device__ __forceinline__
 #else
-#define GB_HD inline
+#define GB_HOST_DEVICE inline
 #endif
 
 namespace gb {
@@ -17,7 +17,7 @@ using append_count = unsigned long long;
 
 // Slot of entry k of an append that got the counter value `first`, or -1 when
 // it does not fit `cap` entries.
-GB_HD long long append_slot(append_count first, unsigned k, long long cap) {
+GB_HOST_DEVICE long long append_slot(append_count first, unsigned k, long long cap) {
   const append_count at = first + k;
   return at < (append_count)(cap > 0 ? cap : 0) ? (long long)at : -1;
 }

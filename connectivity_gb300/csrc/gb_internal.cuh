@@ -304,6 +304,25 @@ struct SmallDesc {
   const int32_t* dst;
   int32_t* adj_scratch;
   int32_t* labels;          // n outputs: smallest member id per component
+  // SCC of a list in host memory, which the caller could write under the call:
+  // 2m ints that keep the pairs as the counting pass read them (null: device
+  // lists).  The scatter reads those, so it fills exactly the slots that were
+  // counted, with ids that were checked.
+  int32_t* kept;
+  GB_HOST_DEVICE void keep(int64_t e, int32_t a, int32_t b) const {
+    if (kept == nullptr) return;
+    kept[e] = a;
+    kept[m + e] = b;
+  }
+  GB_HOST_DEVICE SmallDesc again() const {  // the list of the passes after the first
+    SmallDesc d = *this;
+    if (kept != nullptr) {
+      d.src = kept;
+      d.dst = kept + m;
+      d.id_base = 0;
+    }
+    return d;
+  }
 };
 // Dynamic shared memory of a block for graphs of at most max_n vertices
 // (kind as for launch_small).
