@@ -30,10 +30,10 @@
 // larger root under the smaller, so each root is its component's smallest
 // id; no fixed-point loop.
 //
-// Frontier steps of the general way are edge-balanced: the frontier's degrees are scanned, and
-// thread t takes edges t, t + 1024, ... of the concatenated edge lists,
-// finding its vertex by a binary search over the scan, so a hub's edges are
-// spread over the whole block.
+// Frontier steps of the general way are edge-balanced: the frontier's degrees
+// are scanned, and thread t takes edges t, t + 1024, ... of the concatenated
+// edge lists, finding its vertex by a binary search over the scan, so a hub's
+// edges are spread over the whole block.
 //
 // The CSR comes either from the caller (a device graph or a batch union,
 // whose ids are offset by id_base) or from an edge list, counted and
@@ -279,8 +279,21 @@ __device__ __forceinline__ void uf_unite(int32_t* p, int32_t a, int32_t b) {
 //   - the edges between the vertices left are listed, and those without both
 //     an in- and an out-edge among them labelled;
 //   - what remains is contracted (con_solve).
-// A rest too large for the contraction goes to the colour rounds.
+// A rest too large for the contraction goes to the general way's trim and
+// colour rounds, and searches that go on for long leave everything to it: a
+// pass over all vertices per hop is then the slower way.  R-MAT graphs of this
+// size end within 7 passes.  A pass takes 1.05 us per 1,024 vertices, a hop of
+// a chain in the trim 1.9 us, so up to 1,024 vertices the passes win as long as
+// what they leave fits the contraction; in larger graphs they stop after
+// kHubWork turns of 1,024 vertices (at least kHubPasses).  600 vertices with a
+// hub and a chain of k behind them (start to end, us):
+//     k                     60    300    600   2000   5000
+//     general way only     180    612   1164   3711   9267
+//     no bound, no trim    122    437   5747  23289 102648
+//     with both            125    446   1177   3708   9306
 constexpr int32_t kHubDeg = 16;
+constexpr int32_t kHubPasses = 8;
+constexpr int32_t kHubWork = 32;
 constexpr int32_t kSigAfterSmall = 4;  // colour rounds of colour_mode 2
 
 // One pass of a search from below for vertex v of this lane (valid and not
@@ -336,7 +349,8 @@ struct HubRest {
 
 // SCC of a graph with a hub, up to the vertices that con_solve could not take:
 // their number is returned, their flg is kValid, every other vertex has its
-// label in lab.  Uses kHubSmem bytes of shared memory past the flags.
+// label in lab.  -1: the searches were given up, nothing is labelled.  Uses
+// kHubSmem bytes of shared memory past the flags.
 // (R-MAT graphs leave a few dozen vertices.  Room for 1,024 took enough from
 // the L1 to slow the general path by 7 %, which reads its lists through it.)
 constexpr int32_t kHubVerts = 512, kHubEdges = 1536, kHubLog = 1280;
@@ -366,11 +380,20 @@ __device__ __noinline__ int32_t hub_scc(int n, int32_t pivot, const int32_t* oad
   for (int e = ioff[pivot] + tid; e < ioff[pivot + 1]; e += kST)
     atomicOr(&flg[iadj[e] - base], kBw);
   if (tid == 0) atomicOr(&flg[pivot], kFw | kBw);
+  const int32_t turns = (n + kST - 1) / kST;
   int32_t pass = 0;
   for (bool open = true; open; ++pass) {
-    if (pass >= cap) {
-      ctl[cStop] = 1;
-      return 0;
+    if (pass >= cap) return -1;
+    if (pass >= kHubPasses && pass * turns >= kHubWork) {
+      if (turns > 1) return -1;
+      if (pass == kHubWork) {
+        int32_t most = 0;
+        for (int v = tid; v < n; v += kST) {
+          const uint32_t f = flg[v];
+          if ((f & kValid) && (f & (kFw | kBw)) != (kFw | kBw)) ++most;
+        }
+        if (block_sum(most, ctl) > kHubVerts) return -1;
+      }
     }
     __syncthreads();
     if (tid == 0) qn[0] = 0;
@@ -491,9 +514,10 @@ __device__ __noinline__ int32_t hub_scc(int n, int32_t pivot, const int32_t* oad
 }
 
 // The general path: trim to the fixed point, FW-BW, colour and signature
-// rounds by frontier queues.  nvalid >= 0: only the rounds, for the vertices
-// that hub_scc left.  (Not inlined, as hub_scc is not: with both in the kernel
-// the registers kept across their calls made this path 8 % slower.)
+// rounds by frontier queues.  nvalid >= 0: only the trim and the rounds, for
+// the vertices that hub_scc left.  (Not inlined, as hub_scc is not: with both
+// in the kernel the registers kept across their calls made this path 8 %
+// slower.)
 __device__ __noinline__ void queue_scc(int n, const int32_t* oadj, const int32_t* iadj,
                                        int32_t base, int32_t cap, int32_t colour_rounds,
                                        int32_t nvalid) {
@@ -510,27 +534,36 @@ __device__ __noinline__ void queue_scc(int n, const int32_t* oadj, const int32_t
   int32_t* const pre = s.pre;
   int32_t* const qn = ctl + cQn;
   int cur = 0;
-  if (nvalid < 0) {
   // live degrees without self-loops
+  const bool rest = nvalid >= 0;
   for (int v = tid; v < n; v += kST) {
-    cnt_o[v] = ooff[v + 1] - ooff[v];
-    cnt_i[v] = ioff[v + 1] - ioff[v];
-    flg[v] = kValid;
-    lab[v] = -1;
+    cnt_o[v] = rest ? 0 : ooff[v + 1] - ooff[v];
+    cnt_i[v] = rest ? 0 : ioff[v + 1] - ioff[v];
+    if (!rest) flg[v] = kValid;
+    if (flg[v] & kValid) lab[v] = -1;
   }
   __syncthreads();
-  for_each_edge(n, ooff, oadj, base, [&](int32_t u, int32_t w) {
-    if (u == w) {
-      atomicSub(&cnt_o[u], 1);
-      atomicSub(&cnt_i[u], 1);
-    }
-  });
+  if (rest) {
+    for_each_edge(n, ooff, oadj, base, [&](int32_t u, int32_t w) {
+      if (u != w && (flg[u] & flg[w] & kValid)) {
+        atomicAdd(&cnt_o[u], 1);
+        atomicAdd(&cnt_i[w], 1);
+      }
+    });
+  } else {
+    for_each_edge(n, ooff, oadj, base, [&](int32_t u, int32_t w) {
+      if (u == w) {
+        atomicSub(&cnt_o[u], 1);
+        atomicSub(&cnt_i[u], 1);
+      }
+    });
+  }
   if (tid == 0) qn[0] = 0;
   __syncthreads();
 
   // 1. trim to the fixed point
   for (int v = tid; v < n; v += kST) {
-    if (cnt_o[v] == 0 || cnt_i[v] == 0) {
+    if ((flg[v] & kValid) && (cnt_o[v] == 0 || cnt_i[v] == 0)) {
       flg[v] = 0;
       lab[v] = v;
       push(q[0], &qn[0], v);
@@ -579,7 +612,7 @@ __device__ __noinline__ void queue_scc(int n, const int32_t* oadj, const int32_t
     }
     nvalid = block_sum(cnt, ctl);
     const int32_t pivot = block_argmax(key, id, ctl);
-    if (nvalid > 0 && !ctl[cStop]) {
+    if (!rest && nvalid > 0 && !ctl[cStop]) {
       for (int dir = 0; dir < 2; ++dir) {
         if (tid == 0) {
           flg[pivot] |= dir == 0 ? kFw : kBw;
@@ -629,7 +662,6 @@ __device__ __noinline__ void queue_scc(int n, const int32_t* oadj, const int32_t
       }
       nvalid -= block_sum(cnt2, ctl);
     }
-  }
   }
   __syncthreads();
 
