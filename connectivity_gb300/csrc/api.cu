@@ -96,20 +96,6 @@ gb_status ensure_ws(gb_ctx* c, int32_t n) {
   return GB_OK;
 }
 
-// Grows the context's contraction buffer to m edge pairs per half.
-gb_status ensure_con(gb_ctx* c, int64_t m) {
-  if (m <= c->con_cap) return GB_OK;
-  if (c->con_ws) {
-    cudaStreamSynchronize(c->stream);
-    cudaFree(c->con_ws);
-    c->con_ws = nullptr;
-    c->con_cap = 0;
-  }
-  CK(cudaMalloc(&c->con_ws, (size_t)m * 16), "contraction buffer");
-  c->con_cap = m;
-  return GB_OK;
-}
-
 void fill_params(const gb_opts* o, gb::RunParams& p) {
   gb_opts d;
   gb_opts_default(&d);
@@ -192,7 +178,7 @@ gb_status graph_hints(gb_ctx* c, gb_graph* g) {
   if (!g->symmetric && !g->hint_in)
     CK(dev_alloc((void**)&g->hint_in, hb, true, c->stream), "hint allocation");
   CK(gb::build_hints(g->n, g->m, g->out_off, g->out_adj, g->in_off, g->in_adj, g->hint_out, g->hint_in,
-                     &g->max_deg, c->stream),
+                     g->max_deg, c->stream),
      "hints");
   return GB_OK;
 }
@@ -379,7 +365,7 @@ gb_status run_small(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t* lab
 // passes keeps the searches, which report the cap.
 constexpr int64_t kUnionMaxDeg = 64;
 bool use_union_cc(const gb_graph* g, const gb_opts* o) {
-  if (g->max_deg < 0 || g->max_deg > kUnionMaxDeg) return false;
+  if (g->max_deg[0] < 0 || g->max_deg[0] > kUnionMaxDeg) return false;
   if (o && (!o->canonical || o->fwbw_rounds > 1 || o->expand_mode == 1 ||
             (o->max_steps > 0 && o->max_steps < 3)))
     return false;
@@ -477,15 +463,6 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
   gb::RunParams p{};
   fill_params(o, p);
   p.count_unassigned = st != nullptr ? 1 : 0;
-  // Sparse graphs (up to five edges per vertex: lattices and road networks)
-  // may be contracted; the run kernel decides once it has seen the degrees.
-  // Denser graphs have hubs or short paths, where the searches are better.
-  if (kind == gb::kSCC && bv == nullptr && p.canonical && p.colour_mode == 2 && g->m > 0 &&
-      g->m <= 5 * (int64_t)g->n && p.fwbw_rounds == 1 && p.tune.expand_mode == 0) {
-    if ((s = ensure_con(c, g->m)) != GB_OK) return s;
-    w.con_edges = c->con_ws;
-    w.con_cap = g->m;  // (not what an earlier graph left: the result's route is this graph's)
-  }
   int grid = c->grid;
   if (o && o->grid_blocks > 0 && o->grid_blocks < grid) grid = o->grid_blocks;
   gb::GraphView gv{};
@@ -514,8 +491,28 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
     fills.add(bv->gmin, (size_t)bv->count * 4, 0x7f7f7f7fu);
   }
   CK(gb::launch_fills(fills, sm), "kernel launch");
+  // Sparse graphs (up to five edges per vertex: lattices and road networks)
+  // may be contracted; the run kernel decides once it has seen the degrees.
+  // Denser graphs have hubs or short paths, where the searches are better, and
+  // a hub that the hint build has seen is turned away here already.  The 16
+  // bytes per edge come from the pool for this run only; where they cannot be
+  // had the searches do without.
+  void* con = nullptr;
+  if (kind == gb::kSCC && bv == nullptr && p.canonical && p.colour_mode == 2 && g->m > 0 &&
+      g->m <= 5 * (int64_t)g->n && p.fwbw_rounds == 1 && p.tune.expand_mode == 0 &&
+      g->max_deg[1] <= gb::kConDegree) {
+    if (cudaMallocAsync(&con, (size_t)g->m * 16, c->stream) == cudaSuccess) {
+      w.con_edges = static_cast<unsigned long long*>(con);
+      w.con_cap = g->m;
+    } else {
+      cudaGetLastError();
+      con = nullptr;
+    }
+  }
   c->runs++;
-  CK(gb::launch_run(gv, kind, p, w, grid, sm, ev), "kernel launch");
+  const cudaError_t run_e = gb::launch_run(gv, kind, p, w, grid, sm, ev);
+  if (con) cudaFreeAsync(con, sm);
+  CK(run_e, "kernel launch");
   CK(gb::launch_latch(c->d_ctl, c->d_sticky, sm, c->h_ctl, wait), "kernel launch");
   if (bv != nullptr) CK(gb::launch_localize(w.label, g->n, bv->gid, bv->vbase, sm), "localize");
   if (!dev_labels)
@@ -663,7 +660,6 @@ gb_status gb_ctx_destroy(gb_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   cudaFree(c->ws);
-  cudaFree(c->con_ws);
   cudaFree(c->d_ctl);
   cudaFree(c->d_sticky);
   cudaFree(c->d_tphase);

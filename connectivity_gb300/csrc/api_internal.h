@@ -19,8 +19,6 @@ struct gb_ctx {
   int32_t cap_n = -1;           // workspace capacity in vertices
   void* ws = nullptr;
   gb::Work w{};
-  unsigned long long* con_ws = nullptr;  // contraction's edge pairs (2 x con_cap)
-  int64_t con_cap = 0;
   gb::Ctl* d_ctl = nullptr;
   gb::Ctl* h_ctl = nullptr;     // pinned; behind it h_small
   int32_t* h_small = nullptr;   // kSmallMaxN labels, written by the one-block kernel
@@ -46,7 +44,9 @@ struct gb_graph {
   int32_t* in_adj = nullptr;
   int32_t* hint_out = nullptr;  // pull hints (null for the drop-in staging graph)
   int32_t* hint_in = nullptr;
-  int64_t max_deg = -1;         // largest total degree, found with the hints (-1: not known)
+  // found with the hints (-1: not known): the largest total degree, and the
+  // largest degree on one side of a vertex with edges on both
+  int64_t max_deg[2] = {-1, -1};
   bool pooled = false;          // arrays from the stream-ordered pool
   cudaStream_t pool_stream = nullptr;
 };

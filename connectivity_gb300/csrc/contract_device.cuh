@@ -682,7 +682,6 @@ __device__ __noinline__ bool contract_run(const Contract& k, const Src& src, Ctl
 
 // Out-edges of the valid vertices (E_0 of a device graph): a lane per
 // vertex, whose degree is at most kConDegree.
-constexpr int32_t kConDegree = 32;
 struct ConCsr {
   Csr out;
   const int32_t* list;

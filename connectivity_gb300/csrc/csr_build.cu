@@ -592,23 +592,27 @@ __device__ __forceinline__ uint8_t degree_key(long long d) {
   return (uint8_t)(32 + 8 * (e - 5) + (int)((dd >> (e - 3)) & 7));
 }
 
-// (and the largest total degree, into *most: one atomic per warp)
+// (and the largest total degree, into most[0], and the largest degree on one
+// side among the vertices with edges on both, into most[1]: an atomic of each
+// per warp at most)
 __global__ void k_degree_key(int32_t n, const int64_t* out_off, const int64_t* in_off,
                              uint8_t* key, unsigned long long* most) {
-  long long best = 0;
+  long long best[2] = {0, 0};
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
        v += (int64_t)gridDim.x * blockDim.x) {
-    long long d = out_off[v + 1] - out_off[v];
-    if (in_off) d += in_off[v + 1] - in_off[v];
-    key[v] = degree_key(d);
-    best = d > best ? d : best;
+    const long long dout = out_off[v + 1] - out_off[v];
+    const long long din = in_off ? in_off[v + 1] - in_off[v] : 0;
+    key[v] = degree_key(dout + din);
+    best[0] = max(best[0], dout + din);
+    if (!in_off || (dout > 0 && din > 0)) best[1] = max(best[1], max(dout, din));
   }
-  for (int o = 16; o; o >>= 1) {
-    const long long x = __shfl_xor_sync(0xffffffffu, best, o);
-    best = x > best ? x : best;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    for (int o = 16; o; o >>= 1) best[k] = max(best[k], __shfl_xor_sync(0xffffffffu, best[k], o));
+    if ((threadIdx.x & 31) == 0 &&
+        (unsigned long long)best[k] > *(volatile unsigned long long*)(most + k))
+      atomicMax(most + k, (unsigned long long)best[k]);
   }
-  if ((threadIdx.x & 31) == 0 && (unsigned long long)best > *(volatile unsigned long long*)most)
-    atomicMax(most, (unsigned long long)best);
 }
 
 // The pull hint of a vertex: its neighbour of largest degree key, the first
@@ -656,7 +660,9 @@ struct HintSide {
 };
 
 // The lists the first pass fills.  count: [0] middle vertices, [1] heavy
-// vertices (ordinals), [2] heavy chunks, [3] the largest total degree.
+// vertices (ordinals), [2] heavy chunks, [3] and [4] the largest degrees
+// (k_degree_key).
+constexpr int kHintCounts = 5;
 struct HintLists {
   int32_t* mid;
   int32_t* heavy;                // tag of each heavy ordinal
@@ -1147,8 +1153,8 @@ cudaError_t launch_fills(const Fills& f, cudaStream_t s) {
 
 cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int32_t* out_adj,
                         const int64_t* in_off, const int32_t* in_adj, int32_t* hint_out,
-                        int32_t* hint_in, int64_t* max_deg, cudaStream_t s) {
-  *max_deg = 0;
+                        int32_t* hint_in, int64_t max_deg[2], cudaStream_t s) {
+  max_deg[0] = max_deg[1] = 0;
   if (n <= 0) return cudaSuccess;
   // the sides to build, the out-side first
   HintSide sd[2];
@@ -1157,7 +1163,7 @@ cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int3
   if (in_off && hint_in) sd[sides++] = HintSide{in_off, in_adj, hint_in};
   if (sides == 0) return cudaSuccess;
   if (sides == 1) sd[1] = sd[0];
-  // Scratch: the heavy slots and the three counts (zeroed together), the
+  // Scratch: the heavy slots and the counts (zeroed together), the
   // chunks, the middle list (a vertex-side each at most), the heavy tags,
   // then the degree keys (n bytes).  A side holds m entries, so at most
   // 2m / (kHintWarp + 1) vertex-sides are heavy and their lists make at most
@@ -1166,7 +1172,7 @@ cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int3
   HintLists L;
   L.heavy_cap = std::min<int64_t>(2 * (int64_t)n, 2 * mm / (kHintWarp + 1) + 1);
   L.chunk_cap = 2 * mm / kHintChunk + L.heavy_cap;
-  const size_t zero_b = ((size_t)L.heavy_cap + 4) * 8;
+  const size_t zero_b = ((size_t)L.heavy_cap + kHintCounts) * 8;
   const size_t bytes = zero_b + (size_t)L.chunk_cap * 8 + (size_t)2 * n * 4 +
                        (size_t)L.heavy_cap * 4 + (size_t)n;
   char* buf = nullptr;
@@ -1174,7 +1180,7 @@ cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int3
   if (e != cudaSuccess) return e;
   L.slot = reinterpret_cast<unsigned long long*>(buf);
   L.count = L.slot + L.heavy_cap;
-  L.chunk = reinterpret_cast<int64_t*>(L.count + 4);
+  L.chunk = reinterpret_cast<int64_t*>(L.count + kHintCounts);
   L.mid = reinterpret_cast<int32_t*>(L.chunk + L.chunk_cap);
   L.heavy = L.mid + 2 * (size_t)n;
   uint8_t* deg = reinterpret_cast<uint8_t*>(L.heavy + L.heavy_cap);
@@ -1193,12 +1199,12 @@ cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int3
   k_hint_mid<<<gw_mid, kHintBlock, 0, s>>>(sd[0], sd[1], deg, L.mid, L.count);
   k_hint_heavy<<<gw_heavy, kHintBlock, 0, s>>>(sd[0], sd[1], deg, L);
   k_hint_slots<<<grid_for(L.heavy_cap), 256, 0, s>>>(sd[0], sd[1], L);
-  unsigned long long most = 0;
-  e = cudaMemcpyAsync(&most, L.count + 3, 8, cudaMemcpyDeviceToHost, s);
+  unsigned long long most[2] = {0, 0};
+  e = cudaMemcpyAsync(most, L.count + 3, sizeof(most), cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(buf, s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  *max_deg = e == cudaSuccess ? (int64_t)most : -1;
+  for (int k = 0; k < 2; ++k) max_deg[k] = e == cudaSuccess ? (int64_t)most[k] : -1;
   return e;
 }
 

@@ -58,6 +58,7 @@ enum Stat : int {
 };
 
 constexpr int kConRounds = 64;  // cap on the contraction rounds of a run
+constexpr int32_t kConDegree = 32;  // largest degree on a side of a vertex it takes
 
 struct Ctl {
   // grid barrier word: arrivals so far (low 32 bits, never reset within a
@@ -394,11 +395,12 @@ cudaError_t launch_localize(int32_t* labels, int32_t n, const int32_t* gid, cons
                             cudaStream_t s);
 // Pull hints: for every vertex, its neighbour of largest degree key (the
 // total degree, above 32 rounded down to eight steps per power of two) in
-// each CSR of m entries (hint_in may be null when in_off is).  *max_deg: the
-// largest total degree.  Synchronises the stream.
+// each CSR of m entries (hint_in may be null when in_off is).  max_deg[0]: the
+// largest total degree; [1]: the largest degree on one side among the vertices
+// with edges on both sides.  Synchronises the stream.
 cudaError_t build_hints(int32_t n, int64_t m, const int64_t* out_off, const int32_t* out_adj,
                         const int64_t* in_off, const int32_t* in_adj, int32_t* hint_out,
-                        int32_t* hint_in, int64_t* max_deg, cudaStream_t s);
+                        int32_t* hint_in, int64_t max_deg[2], cudaStream_t s);
 // Seeded R-MAT edge list on the device for n vertices: edge_factor * n
 // candidate edges at scale ceil(log2 n), ids >= n, self-loops and duplicates
 // dropped, sorted by (src, dst); *d_src / *d_dst are cudaMallocAsync'd.
