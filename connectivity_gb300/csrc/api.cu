@@ -1241,14 +1241,14 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   }
   // one stream-ordered allocation: the edges (from host memory, or as the
   // block reads them there), the SCC CSR built by the block (2m ints) and the
-  // labels (for host labels)
+  // union-find's parents, from which host labels are copied
   const bool keep = in_place && kind == gb::kSCC;
   const size_t edge_b = dev_edges && !keep ? 0 : (size_t)m * 8;
   const size_t scr_b = kind == gb::kSCC ? (size_t)m * 8 : 0;  // (the one-block SCC)
-  const size_t lab_b = dev_labels || small ? 0 : (size_t)n * 4;  // (one block: h_small)
+  const size_t par_b = small ? 0 : (size_t)n * 4;
   char* buf = nullptr;
-  if (edge_b + scr_b + lab_b > 0)
-    CK(cudaMallocAsync((void**)&buf, edge_b + scr_b + lab_b, sm), "edge staging");
+  if (edge_b + scr_b + par_b > 0)
+    CK(cudaMallocAsync((void**)&buf, edge_b + scr_b + par_b, sm), "edge staging");
   gb::SmallDesc sd{};
   sd.n = n;
   sd.m = m;
@@ -1265,9 +1265,8 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   }
   if (keep) sd.kept = reinterpret_cast<int32_t*>(buf);
   sd.adj_scratch = scr_b ? reinterpret_cast<int32_t*>(buf + edge_b) : nullptr;
-  sd.labels = dev_labels ? labels
-              : small    ? c->h_small
-                         : reinterpret_cast<int32_t*>(buf + edge_b + scr_b);
+  int32_t* const parent = par_b ? reinterpret_cast<int32_t*>(buf + edge_b + scr_b) : nullptr;
+  sd.labels = dev_labels ? labels : small ? c->h_small : parent;
   const int32_t max_steps = o->max_steps > 0 ? o->max_steps : (1 << 30);
   if (small) {
     if (e == cudaSuccess)
@@ -1276,12 +1275,14 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   } else {
     if (e == cudaSuccess) e = cudaMemsetAsync(&c->d_ctl->err, 0, 2 * sizeof(int), sm);
     if (e == cudaSuccess)
-      e = gb::cc_union_edges(n, m, sd.src, sd.dst, sd.labels, &c->d_ctl->err, sm);
-    if (e == cudaSuccess && !dev_labels)
-      e = cudaMemcpyAsync(labels, sd.labels, (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
+      e = gb::cc_union_edges(n, m, sd.src, sd.dst, parent, sd.labels, &c->d_ctl->err, sm);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(&c->h_ctl->err, &c->d_ctl->err, 2 * sizeof(int), cudaMemcpyDeviceToHost,
                           sm);
+    // (a refused list leaves the caller's labels alone)
+    if (e == cudaSuccess && !dev_labels && (e = cudaStreamSynchronize(sm)) == cudaSuccess &&
+        c->h_ctl->err == 0)
+      e = cudaMemcpyAsync(labels, parent, (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
   }
   if (buf) cudaFreeAsync(buf, sm);
   const cudaError_t e2 = cudaStreamSynchronize(sm);

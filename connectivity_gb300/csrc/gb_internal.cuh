@@ -380,13 +380,14 @@ cudaError_t cc_sampled_device(int32_t n, const int64_t* out_off, const int32_t* 
                               int* d_bad, int* d_err, cudaStream_t s);
 // Weakly connected components by union-find (unionfind.cu), smallest ids as
 // labels (device, n): of a device CSR (a directed graph's out-lists, or a
-// symmetric CSR), and of an edge list (*d_bad |= 1 on an id outside [0, n),
-// whose edge is left out).  Do not wait.
+// symmetric CSR), and of an edge list (*d_bad |= 1 on an id outside [0, n); the
+// labels are then not written, unless they are the parents, n ints of scratch,
+// themselves).  Do not wait.
 // (d_cross: a zeroed word of scratch.)
 cudaError_t cc_union_csr(int32_t n, int64_t m, const int64_t* off, const int32_t* adj,
                          int32_t* labels, unsigned long long* d_cross, cudaStream_t s);
 cudaError_t cc_union_edges(int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
-                           int32_t* labels, int* d_bad, cudaStream_t s);
+                           int32_t* parent, int32_t* labels, int* d_bad, cudaStream_t s);
 // *d_bad |= 1 when an id of adj[0, count) is outside [0, n).  Does not wait.
 cudaError_t check_ids_flag(int32_t n, const int32_t* adj, int64_t count, int* d_bad,
                            cudaStream_t s);

@@ -202,10 +202,11 @@ __global__ void k_uf_edges(int32_t n, int64_t m, int64_t stride, const int32_t* 
 // Every vertex to its root (no join runs at the same time), four vertices per
 // thread with their loads together.  The walk halves no paths: a late halving
 // write would put back a parent that is no root.  Does nothing when cross is
-// given and *cross < least.
+// given and *cross < least, or bad is given and set.  The roots go to out too
+// where that is another array.
 __global__ void k_uf_roots(int32_t n, int32_t* parent, const unsigned long long* cross,
-                           unsigned long long least) {
-  if (cross != nullptr && *cross < least) return;
+                           unsigned long long least, int32_t* out, const int* bad) {
+  if ((cross != nullptr && *cross < least) || (bad != nullptr && *bad != 0)) return;
   constexpr int kU = 4;
   const int64_t nth = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nth * kU) {
@@ -223,6 +224,7 @@ __global__ void k_uf_roots(int32_t n, int32_t* parent, const unsigned long long*
         p[q] = __ldcg(parent + r[q]);
       }
       if (moved) parent[i + q * nth] = r[q];
+      if (out != parent) out[i + q * nth] = r[q];
     }
   }
 }
@@ -263,17 +265,18 @@ cudaError_t cc_union_csr(int32_t n, int64_t m, const int64_t* off, const int32_t
     // vertices, 3 M edges: 0.74 ms instead of 0.51).
     const unsigned long long most = (unsigned long long)m / 4 + 65536;
     k_uf_cross<<<blocks, kUT, 0, s>>>(n, (int32_t)range, kUSample, off, adj, labels, d_cross, most);
-    k_uf_roots<<<uf_grid(n / 4 + 1), 256, 0, s>>>(n, labels, d_cross, most);
+    k_uf_roots<<<uf_grid(n / 4 + 1), 256, 0, s>>>(n, labels, d_cross, most, labels, nullptr);
     k_uf_cross<<<blocks, kUT, 0, s>>>(n, (int32_t)range, 1, off, adj, labels, d_cross, 0ull);
-    k_uf_roots<<<uf_grid(n / 4 + 1), 256, 0, s>>>(n, labels, nullptr, 0ull);
+    k_uf_roots<<<uf_grid(n / 4 + 1), 256, 0, s>>>(n, labels, nullptr, 0ull, labels, nullptr);
   }
   return cudaGetLastError();
 }
 
 cudaError_t cc_union_edges(int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
-                           int32_t* labels, int* d_bad, cudaStream_t s) {
+                           int32_t* parent, int32_t* labels, int* d_bad, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_uf_self<<<uf_grid(n), 256, 0, s>>>(n, labels);
+  if (m == 0) parent = labels;
+  k_uf_self<<<uf_grid(n), 256, 0, s>>>(n, parent);
   if (m > 0) {
     // A few joins first, then ever more with the parents flattened in between:
     // most edges of the later parts find equal parents at the first load.
@@ -282,9 +285,12 @@ cudaError_t cc_union_edges(int32_t n, int64_t m, const int32_t* src, const int32
     int64_t stride = 1;
     while (m / stride > kULast) stride *= kUSample;
     for (; stride >= 1; stride /= kUSample) {
-      k_uf_edges<<<uf_grid((m / stride + 3) / 4), 256, 0, s>>>(n, m, stride, src, dst, labels,
+      k_uf_edges<<<uf_grid((m / stride + 3) / 4), 256, 0, s>>>(n, m, stride, src, dst, parent,
                                                               d_bad);
-      k_uf_roots<<<uf_grid(n / 4 + 1), 256, 0, s>>>(n, labels, nullptr, 0ull);
+      // (the last part has read every id: only then may the labels be written)
+      const bool last = stride == 1;
+      k_uf_roots<<<uf_grid(n / 4 + 1), 256, 0, s>>>(n, parent, nullptr, 0ull,
+                                                    last ? labels : parent, last ? d_bad : nullptr);
     }
   }
   return cudaGetLastError();

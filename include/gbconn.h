@@ -331,7 +331,8 @@ gb_status gb_cc(gb_ctx* ctx, const gb_graph* g, int32_t* labels, const gb_opts* 
  * memory and scratch from the stream-ordered pool: one launch, no radix
  * sort.  WCC of a larger list is a union-find over the edges; for SCC it is
  * built as a device graph, run and freed.  Waits
- * for the result.  GB_ERR_INVALID: an id outside [0, n). */
+ * for the result.  GB_ERR_INVALID: an id outside [0, n); the labels are then
+ * left as they were. */
 gb_status gb_scc_edges(gb_ctx* ctx, int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
                        int32_t* labels, const gb_opts* opts);
 gb_status gb_wcc_edges(gb_ctx* ctx, int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
