@@ -986,6 +986,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
   }
 
   // ---- SCC ----------------------------------------------------------------
+  __syncthreads();  // the offsets, from here on read across threads
   int32_t nvalid = -1;
   int32_t hub = -1;
   if (colour_rounds == kSigAfterSmall) {
@@ -993,7 +994,6 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
     // both sides
     long long key = -1;
     int32_t id = 0x7fffffff;
-    __syncthreads();  // the offsets
     for (int v = tid; v < n; v += kST) {
       const int32_t od = ooff[v + 1] - ooff[v], idg = ioff[v + 1] - ioff[v];
       const long long k = (long long)od * (long long)idg;
