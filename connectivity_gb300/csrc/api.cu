@@ -361,13 +361,13 @@ gb_status run_small(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t* lab
 // uniform random graphs too (1 M vertices, 3 M edges: 1.78 ms against 0.51;
 // with 4 M edges they take 0.36 and the union-find 0.75).  With hubs the
 // union-find loses (R-MAT of 1 M vertices and 4 edges each: 4.5 ms against
-// 0.28: the hubs' lists meet in a few blocks).  max_steps below the union-find's three
-// passes keeps the searches, which report the cap.
+// 0.28: the hubs' lists meet in a few blocks).  A step cap that the searches
+// could meet keeps them.
 constexpr int64_t kUnionMaxDeg = 64;
 bool use_union_cc(const gb_graph* g, const gb_opts* o) {
   if (g->max_deg[0] < 0 || g->max_deg[0] > kUnionMaxDeg) return false;
   if (o && (!o->canonical || o->fwbw_rounds > 1 || o->expand_mode == 1 ||
-            (o->max_steps > 0 && o->max_steps < 3)))
+            (o->max_steps > 0 && !gb::steps_free(o->max_steps, g->n))))
     return false;
   return g->m < (g->symmetric ? 8 : 4) * (int64_t)g->n;
 }
@@ -463,6 +463,7 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
   gb::RunParams p{};
   fill_params(o, p);
   p.count_unassigned = st != nullptr ? 1 : 0;
+  p.free_steps = gb::steps_free(p.tune.max_steps, g->n) ? 1 : 0;
   int grid = c->grid;
   if (o && o->grid_blocks > 0 && o->grid_blocks < grid) grid = o->grid_blocks;
   gb::GraphView gv{};
@@ -500,7 +501,7 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
   void* con = nullptr;
   if (kind == gb::kSCC && bv == nullptr && p.canonical && p.colour_mode == 2 && g->m > 0 &&
       g->m <= 5 * (int64_t)g->n && p.fwbw_rounds == 1 && p.tune.expand_mode == 0 &&
-      g->max_deg[1] <= gb::kConDegree) {
+      p.free_steps && g->max_deg[1] <= gb::kConDegree) {
     if (cudaMallocAsync(&con, (size_t)g->m * 16, c->stream) == cudaSuccess) {
       w.con_edges = static_cast<unsigned long long*>(con);
       w.con_cap = g->m;
@@ -1212,10 +1213,10 @@ gb_status run_edges(gb_ctx* c, gb::RunKind kind, int32_t n, int64_t m, const int
   if (!o) o = gb::class_opts(c, n);
   if (!o) o = &d;
   const bool small = n <= gb::kSmallMaxN && m < (1ll << 31) && o->small_path && o->canonical;
-  // WCC of a larger list: union-find over the edges, no CSR (its three
-  // passes against the step cap as in use_union_cc)
+  // WCC of a larger list: union-find over the edges, no CSR (the step cap as
+  // in use_union_cc)
   const bool uni = !small && kind == gb::kWCC && o->canonical &&
-                   !(o->max_steps > 0 && o->max_steps < 3);
+                   (o->max_steps <= 0 || gb::steps_free(o->max_steps, n));
   if (!small && !uni) {
     gb_graph* g = nullptr;
     gb_status s = gb::graph_from_edges(c, n, m, src, dst, true, true, &g);

@@ -609,12 +609,12 @@ __device__ __noinline__ int con_solve(const Src& src, int32_t n, int32_t* smem,
 }
 
 // The tail: block 0 finishes the graph of round t (at most kConTailVerts
-// vertices and kConTailEdges edges) and leaves a component in tc for every
-// vertex of A_t.
+// vertices and kConTailEdges edges) and leaves a component or kConOpen in tc
+// for every vertex of A_t.
 constexpr int32_t kConTailBytes = con_bytes(kConTailVerts, kConTailEdges, kConTailLog);
 static_assert(kConTailBytes + kConTailVerts * 4 <= kDynSmem,
               "the tail's arrays fit the dynamic shared memory");
-__device__ __forceinline__ void con_tail(const Contract& k, Ctl* c, int t, int32_t steps_left,
+__device__ __forceinline__ void con_tail(const Contract& k, int t, int32_t steps_left,
                                          int32_t* smem, int32_t* rounds) {
   __shared__ int s_left;
   int32_t* const gid = smem + kConTailBytes / 4;
@@ -630,8 +630,8 @@ __device__ __forceinline__ void con_tail(const Contract& k, Ctl* c, int t, int32
   int32_t* comp;
   const int u = con_solve<kConTailVerts, kConTailEdges, kConTailLog>(ConLocal{&k, t}, n, smem,
                                                                      &s_left, &comp);
+  // (out of steps, all of it is left to the rounds, which have a cap of their own)
   const bool ok = s_left >= 0;
-  if (!ok && tid == 0) set_err(c, kErrIterLimit, 431);
   for (int i = tid; i < n; i += nth) {
     const int32_t x = ok ? comp[i] : kConOpen;
     k.tc[gid[i]] = x < 0 ? kConOpen : gid[x];
@@ -671,7 +671,7 @@ __device__ __noinline__ bool contract_run(const Contract& k, const Src& src, Ctl
     con_open(k, g, t, undone);
   } else if (small) {
     trace_rec(c, __ldcg(k.cntA + t), 23);
-    if (blockIdx.x == 0) con_tail(k, c, t, max_steps - (st.s - st.s0), smem, rounds);
+    if (blockIdx.x == 0) con_tail(k, t, max_steps - (st.s - st.s0), smem, rounds);
   }
   trace_rec(c, t, 24);
   if (!g.sync(430)) return false;

@@ -205,6 +205,16 @@ struct GraphView {
 // Kind of run.
 enum RunKind : int { kSCC = 0, kWCC = 1 };
 
+// Whether a step cap is too high for the searches and rounds of a graph of n
+// vertices to meet.  The shorter ways (contraction, residual phase, union-find,
+// the one-block searches from a hub) count other steps, so a cap that may be
+// met keeps the phases it was made for: it then stops the calls that it always
+// stopped, and no others.
+GB_HOST_DEVICE bool steps_free(int64_t max_steps, int64_t n) {
+  const int64_t most = 2 * n + 4096;
+  return max_steps >= (most < (1 << 30) ? most : (1 << 30));
+}
+
 struct RunParams {
   int32_t trim_level;     // 0: none, 1: one pass, 2: fixed point
   int32_t trim_pairs;     // 1: size-2 components leave with the trim
@@ -212,6 +222,7 @@ struct RunParams {
   int32_t canonical;      // 1: relabel with the minimum member id
   int32_t pivot_hint;     // >= 0: use as FW-BW source if still valid
   int32_t count_unassigned;  // 1: a final pass counts labels outside [0, n)
+  int32_t free_steps;     // 1: steps_free(tune.max_steps, n)
   int32_t colour_mode;    // SCC: 0 colour rounds, 1 signature rounds, 2 the
                           // signature rounds from kSigMin residual vertices
   Tune tune;

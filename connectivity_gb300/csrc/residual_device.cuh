@@ -170,7 +170,7 @@ __device__ __noinline__ bool residual_phase(const Args& A, Smem& sm) {
     if (b == 0) {
       __shared__ int s_open;
       if (t == 0) s_open = 0;
-      con_tail(k, c, 1, A.p.tune.max_steps - (st.s - st.s0), sm.stage_base, &c->ncolour_rounds);
+      con_tail(k, 1, A.p.tune.max_steps - (st.s - st.s0), sm.stage_base, &c->ncolour_rounds);
       __syncthreads();
       for (int i = t; i < na; i += blockDim.x) {
         const int32_t v = __ldcg(k.A[1] + i), cv = __ldcg(k.tc + v);

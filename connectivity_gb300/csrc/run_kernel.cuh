@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_run(Args A) {
   const bool scc = A.kind == kSCC;
   bool left = true;
   if constexpr (NC == 1) {
-    if (scc && A.p.colour_mode == 2) {
+    if (scc && A.p.colour_mode == 2 && A.p.free_steps) {
       left = residual_phase(A, sm);
       if (left && !grid_barrier(c, 905)) return;
     }

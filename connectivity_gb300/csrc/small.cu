@@ -493,10 +493,7 @@ __device__ __noinline__ int32_t hub_scc(int n, int32_t pivot, const int32_t* oad
   con_solve<kHubVerts, kHubEdges, kHubLog>(HubRest{edges, qn[1], lab}, left, tail, ctl + cLeft,
                                            &comp);
   __syncthreads();
-  if (ctl[cLeft] < 0) {
-    ctl[cStop] = 1;
-    return 0;
-  }
+  if (ctl[cLeft] < 0) return left;  // (out of steps: all of it is left to the rounds)
   int32_t* const small = tail;  // (the contraction's edges are done with)
   for (int i = tid; i < left; i += kST) small[i] = 0x7fffffff;
   __syncthreads();
@@ -989,7 +986,7 @@ __global__ void __launch_bounds__(kST, 1) k_small(SmallDesc one, const SmallDesc
   __syncthreads();  // the offsets, from here on read across threads
   int32_t nvalid = -1;
   int32_t hub = -1;
-  if (colour_rounds == kSigAfterSmall) {
+  if (colour_rounds == kSigAfterSmall && steps_free(max_steps, n)) {
     // the vertex of largest out x in degree, among those with kHubDeg on
     // both sides
     long long key = -1;

@@ -81,7 +81,10 @@ typedef struct gb_opts {
                           edges (15, the reference's ALPHA scc_main.cpp:64) */
   float beta;          /* pull -> push when frontier * beta < candidates
                           (25, the reference's BETA scc_main.cpp:65) */
-  int32_t max_steps;   /* cap on device steps per phase (1 << 30) */
+  int32_t max_steps;   /* cap on device steps per phase (1 << 30).  A cap
+                          below 2 n + 4096 keeps the searches and rounds where
+                          a shorter way would be taken (contraction,
+                          union-find, one-block searches from a hub). */
   int32_t grid_blocks; /* 0: all resident blocks; else a smaller grid */
   int32_t trim_pairs;  /* 1: after the trim, remove size-2 SCCs (two vertices
                           that are each other's only in-neighbour, or only
@@ -137,7 +140,7 @@ typedef struct gb_opts {
                           graph of fewer than 4 n edges (8 n entries of a
                           symmetric CSR) and no vertex of total degree above
                           64 takes a union-find over its edges (canonical = 1,
-                          fwbw_rounds = 1, expand_mode = 0, max_steps >= 3;
+                          fwbw_rounds = 1, expand_mode = 0, max_steps as above;
                           the statistics then hold the times only). */
 } gb_opts;
 
