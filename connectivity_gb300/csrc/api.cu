@@ -362,7 +362,7 @@ gb_status run_small(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t* lab
 // with 4 M edges they take 0.36 and the union-find 0.75).  With hubs the
 // union-find loses (R-MAT of 1 M vertices and 4 edges each: 4.5 ms against
 // 0.28: the hubs' lists meet in a few blocks).  A step cap that the searches
-// could meet keeps them.
+// could meet keeps them, and so does a caller that asks for their statistics.
 constexpr int64_t kUnionMaxDeg = 64;
 bool use_union_cc(const gb_graph* g, const gb_opts* o) {
   if (g->max_deg[0] < 0 || g->max_deg[0] > kUnionMaxDeg) return false;
@@ -446,7 +446,7 @@ gb_status run_graph_impl(gb_ctx* c, const gb_graph* g, gb::RunKind kind, int32_t
   if (bv == nullptr && use_small(g, o)) return run_small(c, g, kind, labels, o, st, wait);
   if (bv == nullptr && kind == gb::kWCC && o && o->wcc_mode == 1)
     return run_union_cc(c, g, labels, st, wait, true);
-  if (bv == nullptr && kind == gb::kWCC && use_union_cc(g, o))
+  if (bv == nullptr && kind == gb::kWCC && st == nullptr && use_union_cc(g, o))
     return run_union_cc(c, g, labels, st, wait, false);
   gb_status s = ensure_ws(c, g->n);
   if (s != GB_OK) return s;

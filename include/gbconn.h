@@ -140,8 +140,8 @@ typedef struct gb_opts {
                           graph of fewer than 4 n edges (8 n entries of a
                           symmetric CSR) and no vertex of total degree above
                           64 takes a union-find over its edges (canonical = 1,
-                          fwbw_rounds = 1, expand_mode = 0, max_steps as above;
-                          the statistics then hold the times only). */
+                          fwbw_rounds = 1, expand_mode = 0, max_steps as above,
+                          no statistics asked for). */
 } gb_opts;
 
 void gb_opts_default(gb_opts* o);
