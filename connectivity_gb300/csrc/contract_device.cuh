@@ -542,11 +542,11 @@ __device__ __forceinline__ bool con_core(const Contract& k, const W& w, int t, v
 // most E; L entries of log.  Afterwards comp[i] (in smem, valid until it is reused)
 // is the component of vertex i, the id of one of its members, or kConOpen
 // when the log ran out.  *left: steps the block may still take; negative
-// afterwards when they ran out (comp is then not set).  Returns the rounds.
+// afterwards when they ran out (comp is then not set).
 constexpr int32_t con_bytes(int32_t V, int32_t E, int32_t L) { return V * 40 + (2 * E + L) * 8; }
 template <int32_t V, int32_t E, int32_t L, class Src>
-__device__ __noinline__ int con_solve(const Src& src, int32_t n, int32_t* smem,
-                                      volatile int* left, int32_t** comp) {
+__device__ __noinline__ void con_solve(const Src& src, int32_t n, int32_t* smem,
+                                       volatile int* left, int32_t** comp) {
   __shared__ int s_flag;
   __shared__ int32_t s_cnt[2][kConRounds + 2];
   __shared__ append_count s_ecnt[2][kConRounds + 2];
@@ -605,7 +605,6 @@ __device__ __noinline__ int con_solve(const Src& src, int32_t n, int32_t* smem,
   }
   __syncthreads();
   for (int x = u - (undone ? 2 : 1); ok && x >= 0; --x) ok = con_undo(l, b, x);
-  return u;
 }
 
 // The tail: block 0 finishes the graph of round t (at most kConTailVerts
@@ -628,15 +627,16 @@ __device__ __forceinline__ void con_tail(const Contract& k, int t, int32_t steps
   }
   __syncthreads();
   int32_t* comp;
-  const int u = con_solve<kConTailVerts, kConTailEdges, kConTailLog>(ConLocal{&k, t}, n, smem,
-                                                                     &s_left, &comp);
+  con_solve<kConTailVerts, kConTailEdges, kConTailLog>(ConLocal{&k, t}, n, smem, &s_left, &comp);
   // (out of steps, all of it is left to the rounds, which have a cap of their own)
   const bool ok = s_left >= 0;
   for (int i = tid; i < n; i += nth) {
     const int32_t x = ok ? comp[i] : kConOpen;
     k.tc[gid[i]] = x < 0 ? kConOpen : gid[x];
   }
-  if (tid == 0) *rounds = t + u;
+  // (all of this is one round to the caller: how many it took depends on the
+  // order in which the vertices were appended)
+  if (tid == 0) *rounds = t + 1;
 }
 
 // The whole contraction: rounds until no vertex is alive or they stop

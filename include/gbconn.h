@@ -159,7 +159,8 @@ typedef struct gb_stats {
   int32_t pivot;          /* FW-BW source, -1 if none */
   int32_t colour_rounds;  /* rounds of the colour phase, or of the contraction
                              that found every component in its place (its time
-                             is part of ms_reach) */
+                             is part of ms_reach; what one block finishes
+                             counts as one round) */
   int64_t n_trim;         /* vertices labelled by trim */
   int64_t n_visit_fw;     /* vertices reached forward from the pivot */
   int64_t n_fwbw;         /* vertices labelled by FW-BW */
