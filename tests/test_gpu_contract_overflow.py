@@ -25,6 +25,16 @@ def _fork(k, f, base=0):
     return base + 7 * k, s.astype(np.int32), d.astype(np.int32)
 
 
+def _ring(k, f, base=0):
+    """k copies of a component that drops a fifth of its edges in the first
+    round and hardly any in the second: u <-> y, u -> v, u -> w, v -> z and
+    w -> z (f edges each), z -> p and z -> r, p <-> q, r <-> t, p -> u, r -> u."""
+    u, y, v, w, z, p, q, r, t = (base + i * k + np.arange(k) for i in range(9))
+    s = np.r_[u, y, u, u, np.repeat(v, f), np.repeat(w, f), z, z, p, q, r, t, p, r]
+    d = np.r_[y, u, v, w, np.repeat(z, f), np.repeat(z, f), p, r, q, p, t, r, u, u]
+    return base + 9 * k, s.astype(np.int32), d.astype(np.int32)
+
+
 def _join(n, s, d, add):
     n2, s2, d2 = add(n)
     return n2, np.r_[s, s2].astype(np.int32), np.r_[d, d2].astype(np.int32)
@@ -50,6 +60,9 @@ CASES = {
     "log_shuffled": _shuffle(*_fork(1500, 10), 3),
     # beside a lattice, which keeps vertices alive
     "log_and_grid": _join(*graphs.grid(40), lambda b: _fork(1500, 10, b)),
+    # 48,000 and 45,000 edges in the first two rounds for 60,000 places
+    "edges": _ring(1500, 14),
+    "edges_shuffled": _shuffle(*_ring(1500, 14), 4),
     # a residual that the one-block tail takes, whose log of 2,560 gets 4,400
     "tail_log": _join(*gb.rmat_edges(14, 16, 3), lambda b: _fork(55, 20, b)),
     # a residual of more edges than its list
