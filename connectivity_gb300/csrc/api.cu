@@ -290,7 +290,7 @@ gb_status finish_run(gb_ctx* c, const gb_graph* g, gb_stats* st) {
 // cost more than the cooperative grid's steps (the line was drawn
 // for SCC by searches in one block: 173 against 220 us at 4,000 vertices and
 // 52,000 edges, 233 against 222 at 6,000 and 73,000.  Graphs with a hub now
-// take 52 us at the former size, graphs without one as long as they did);
+// take 48 us at the former size, graphs without one as long as they did);
 // 2 takes it whenever the graph fits.
 bool use_small(const gb_graph* g, const gb_opts* o) {
   if (g->n > gb::kSmallMaxN || g->m >= (1ll << 31)) return false;

@@ -41,11 +41,14 @@
 //
 // A round shrinks the 1024^2 lattice of the benchmark by a factor of two to
 // three, so about 20 rounds replace some 27,000 dependent hops: 111 ms ->
-// 1.15 ms of device time (2048^2: 2.8 ms; the first round takes a quarter of
-// it, each of the small ones 35 us of grid barriers and dependent L2 reads,
-// the tail in one block 110 us).  A core that no longer shrinks (uniform
-// random graphs of three or more edges per vertex, one-way street lattices)
-// is left to the searches and colour rounds.
+// 1.1 ms of device time (the first round takes a quarter of it, each of the
+// small ones 35 us of grid barriers and dependent L2 reads, the tail in one
+// block 110 us).  When a round drops less than a fifth of the edges before the
+// tail takes the rest, every vertex goes back to the searches and rounds:
+// one-way street lattices, the cores of random graphs, but also lattices of some
+// 2,048 a side (for two seeds in five 2.8 ms becomes 155 ms) and more, and
+// chains of more than some 65,000 vertices numbered in order, where every other
+// pair of rounds runs against the ids.
 #pragma once
 #include "run_device.cuh"
 
